@@ -81,6 +81,7 @@ struct NbgsBuf {
     int32_t *rem = nullptr;                   // uncoloured contacts left after each colouring round
     unsigned int *bar2 = nullptr;             // grid barrier of the colouring rounds
     int32_t *slot_of = nullptr;               // per body: -1, or its claim in the compact sweep
+    bool flow_off = false;                    // the sweep form without barriers cannot be launched
     bool compact_off = false;                 // the compact sweep form cannot be launched
     bool staged_off = false;                  // nor the grid form with staged contacts
     bool on_device = false;                   // the last step's counts are only on the device

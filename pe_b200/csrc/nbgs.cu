@@ -165,6 +165,8 @@ struct Cache {
     T4<T> *p;     // impulse in the contact frame (n, t, o, -)
     T4<T> *dc;    // 2 per contact: Delassus block in the contact frame [xy xz yy yz] [zz - - -]
                   // (its xx is rec[2].w), read by relaxation models 2-5 only
+    int4 *seq;    // place among body 1's contacts, their number, the same for body 2 (0, 0: wall)
+    ulonglong2 *mail;   // per contact and side: the body's corrections for its next update (k_sweeps_flow)
     // the sweeps' accessors
     __device__ __forceinline__ int2 get_ids(int64_t k) const { return ids[k]; }
     __device__ __forceinline__ const T4<T> *rec_of(int64_t k) const { return rec + (int64_t)kRec * k; }
@@ -598,22 +600,23 @@ __global__ void k_color_rounds(const int32_t *ncp, const int32_t *dd, int64_t se
 // both bodies), in one launch.  Where a body carries dozens of contacts (box stacks) this needs
 // about as many colours as the busiest body has contacts, the least possible, where the parallel
 // rounds need a launch pair per round and end with more colours.
-// The used-colour masks live in shared memory when they fit (used_global == null), else in
-// the zeroed global array.
+// The used-colour masks live in shared memory when they fit (in_smem; copied out at the end), else
+// in the zeroed global array.
 template <int W>
 __global__ void k_color_serial(const int32_t *ncp, const int32_t *dd, int64_t serial_max,
                                const int32_t *__restrict__ b1, const int32_t *__restrict__ b2,
                                int32_t *__restrict__ color, int64_t nbod, uint64_t *used_global,
-                               int32_t *err) {
+                               int in_smem, int32_t *err) {
     if (dd[kDdAbort]) return;
     const int64_t nc = *ncp;
     if (nc > serial_max) return;   // the parallel rounds colour this step
     extern __shared__ uint64_t used_shared[];
-    uint64_t *used = used_global ? used_global : used_shared;
-    if (!used_global)
+    uint64_t *used = in_smem ? used_shared : used_global;
+    if (in_smem) {
         for (int64_t i = threadIdx.x; i < nbod * W; i += blockDim.x) used_shared[i] = 0ull;
-    __syncthreads();
-    if (threadIdx.x != 0) return;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
     // the bodies of the next contacts are loaded ahead, off the chain of mask updates
     constexpr int kAhead = 8;
     int32_t qa[kAhead], qb[kAhead];
@@ -647,6 +650,11 @@ __global__ void k_color_serial(const int32_t *ncp, const int32_t *dd, int64_t se
         used[(int64_t)a * W + (col >> 6)] |= 1ull << (col & 63);
         if (b >= 0) used[(int64_t)b * W + (col >> 6)] |= 1ull << (col & 63);
     }
+    }
+    if (!in_smem) return;
+    __syncthreads();
+    // the masks say each contact's place among its bodies' contacts (k_cache)
+    for (int64_t i = threadIdx.x; i < nbod * W; i += blockDim.x) used_global[i] = used_shared[i];
 }
 
 __global__ void k_color_hist(const int32_t *ncp, const int32_t *dd, int32_t *color,
@@ -709,12 +717,42 @@ __global__ void k_color_pos(const int32_t *ncp, const int32_t *dd, const int32_t
 // ---- contact cache (HCSITS.h:1767-1815) --------------------------------------------------------
 template <typename T, bool GEN>
 __global__ void k_cache(const int32_t *ncp, const int32_t *dd, int64_t cap, Raw<T> raw,
-                        const int32_t *pos, BodyV<T> bv, int64_t nb, Cache<T> cc) {
+                        const int32_t *pos, const int32_t *color, const uint64_t *used,
+                        const int32_t *adj_start, int32_t *adj, BodyV<T> bv, int64_t nb, Cache<T> cc) {
     if (dd[kDdAbort]) return;
     const int64_t nc = *ncp;
     GRID_STRIDE(c, nc) {
     const int64_t k = pos[c];
     const int32_t b1 = raw.b1[c], b2 = raw.b2[c];
+    // the contact's place among each of its bodies' contacts in colour order, and their number
+    // (a body has one contact per colour of its mask)
+    {
+        constexpr int W = GEN ? 4 : 1;
+        const int col = color[c];
+        auto place = [&](int32_t b, int &s, int &d) {
+            s = d = 0;
+            if (b < 0) return;
+#pragma unroll
+            for (int wd = 0; wd < W; ++wd) {
+                const uint64_t u = used[(int64_t)b * W + wd];
+                d += __popcll(u);
+                if (col >= 64 * wd + 64) s += __popcll(u);
+                else if (col > 64 * wd) s += __popcll(u & ((1ull << (col - 64 * wd)) - 1ull));
+            }
+        };
+        int4 sq;
+        place(b1, sq.x, sq.y);
+        place(b2, sq.z, sq.w);
+        cc.seq[k] = sq;
+        if (adj) {
+            // the bodies' contacts in colour order, and empty mailboxes
+            if (sq.x < sq.y) adj[adj_start[b1] + sq.x] = (int32_t)(2 * k);
+            if (sq.z < sq.w) adj[adj_start[b2] + sq.z] = (int32_t)(2 * k + 1);
+#pragma unroll
+            for (int q = 0; q < (int)sizeof(T); ++q)   // FlowRec<T>::N vectors for each side
+                cc.mail[2 * ((q >> 1) * cap + k) + (q & 1)] = make_ulonglong2(0ull, 0ull);
+        }
+    }
     const V3<T> r1 = ld3c(raw.r1, c, cap), r2 = ld3c(raw.r2, c, cap), n = ld3c(raw.n, c, cap);
     V3<T> t;
     if (fabs(n.x) < fabs(n.y)) {
@@ -977,63 +1015,144 @@ __device__ __forceinline__ V3<T> solve_gmd(V3<T> pcf, const V3<T> &g, const T D[
     return v3(invA_nn * (-g.x - D[1] * x0 - D[2] * x1), x0, x1);
 }
 
-// one contact of one sweep of relaxation model MODEL (pe's RelaxationModel, HCSITS.h:172-179);
-// COHERENT: read the velocity corrections and the impulse from L2
-template <typename T, int MODEL, bool COHERENT, bool GEN = false, typename BV = BodyV<T>,
-          typename CC = Cache<T>>
-__device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
-                                              const BV &bv, int track_delta,
-                                              unsigned long long *delta) {
-    constexpr bool FRICTION = MODEL != 0;
-    const int2 ids = cc.get_ids(k);
-    const int32_t b1 = ids.x, b2 = ids.y;
-    const T4<T> *R = cc.rec_of(k);
-    const T4<T> q0 = R[0], q1 = R[1], q2 = R[2];
-    const V3<T> n = xyz<T>(q0), r1 = xyz<T>(q1), r2 = xyz<T>(q2);
-    const T dist = q0.w, dn_inv = q1.w;
-    const T4<T> pc4 = cc.template get_p<COHERENT>(k);
-    const V3<T> pc = xyz<T>(pc4);  // contact frame
-    const T4<T> vr1 = bv.get_vr(b1), wr1 = bv.get_wr(b1);
-    const T im1 = vr1.w, ii1 = wr1.w;
-    V3<T> dv1 = xyz<T>(bv.template get_dv<COHERENT>(b1));
-    V3<T> dw1 = xyz<T>(bv.template get_dw<COHERENT>(b1));
-    const V3<T> v1 = xyz<T>(vr1), w1 = xyz<T>(wr1);
-    V3<T> dv2 = v3(T(0), T(0), T(0)), dw2 = dv2, v2 = dv2, w2 = dv2;
-    T im2 = T(0), ii2 = T(0);
-    if (b2 >= 0) {
-        const T4<T> vr2 = bv.get_vr(b2), wr2 = bv.get_wr(b2);
-        im2 = vr2.w;
-        ii2 = wr2.w;
-        dv2 = xyz<T>(bv.template get_dv<COHERENT>(b2));
-        dw2 = xyz<T>(bv.template get_dw<COHERENT>(b2));
-        v2 = xyz<T>(vr2);
-        w2 = xyz<T>(wr2);
+// One body of a contact: its masses, lever arm and predicted velocities, and its corrections.
+template <typename T, bool GEN>
+struct Side {
+    T4<T> vr, wr;      // v, 1/m and w, 1/I
+    InvI<T, GEN> I;
+    V3<T> r, dv, dw;
+    // the velocity a world-frame impulse causes at the contact through this body's rotation
+    __device__ __forceinline__ V3<T> through(const V3<T> &p) const { return cross(I(cross(r, p)), r); }
+};
+
+// The two bodies of a contact, both in one thread (two: body 2 is not a wall; a wall's records
+// and corrections are zero).
+template <typename T, bool GEN>
+struct BothSides {
+    Side<T, GEN> a, b;
+    bool two;
+    __device__ __forceinline__ V3<T> velocity() const {
+        return ((xyz<T>(a.vr) + a.dv) - (xyz<T>(b.vr) + b.dv) + cross(xyz<T>(a.wr) + a.dw, a.r)) -
+               cross(xyz<T>(b.wr) + b.dw, b.r);
     }
-    const InvI<T, GEN> I1 = load_invi<T, GEN>(bv, b1, ii1), I2 = load_invi<T, GEN>(bv, b2, ii2);
-    static_assert(!GEN || std::is_same<BV, BodyV<T>>::value, "full inverse inertias: BodyV only");
+    __device__ __forceinline__ V3<T> through(const V3<T> &p) const { return add_through(p, nullptr); }
+    // (g + body 1's part) + body 2's part (g null: their sum)
+    __device__ __forceinline__ V3<T> add_through(const V3<T> &p, const V3<T> *g) const {
+        const V3<T> e1 = a.through(p);
+        const V3<T> e2 = two ? b.through(p) : v3(T(0), T(0), T(0));
+        return g ? (*g + e1) + e2 : e1 + e2;
+    }
+    __device__ __forceinline__ void remove(const V3<T> &p) {
+        a.dv = a.dv - a.vr.w * p;
+        a.dw = a.dw - a.I(cross(a.r, p));
+        if (two) {
+            b.dv = b.dv + b.vr.w * p;
+            b.dw = b.dw + b.I(cross(b.r, p));
+        }
+    }
+    __device__ __forceinline__ void apply(const V3<T> &p) {
+        a.dv = a.dv + a.vr.w * p;
+        a.dw = a.dw + a.I(cross(a.r, p));
+        if (two) {
+            b.dv = b.dv - b.vr.w * p;
+            b.dw = b.dw - b.I(cross(b.r, p));
+        }
+    }
+};
+
+// The same with one body in each lane of an even and odd pair: half the registers and about half
+// the instructions of an update, with the same operations on the same values.
+template <typename T, bool GEN>
+struct PairedSides {
+    Side<T, GEN> s;
+    bool second;       // this lane holds body 2
+    bool body;         // it is not a wall
+    V3<T> ov, ow;      // what removing the old impulse adds to this body's corrections
+    __device__ __forceinline__ V3<T> other(const V3<T> &v) const {
+        const unsigned int pair = 3u << (threadIdx.x & 30u);
+        return v3(__shfl_xor_sync(pair, v.x, 1), __shfl_xor_sync(pair, v.y, 1), __shfl_xor_sync(pair, v.z, 1));
+    }
+    __device__ __forceinline__ V3<T> velocity() const {
+        const V3<T> v = xyz<T>(s.vr) + s.dv, c = cross(xyz<T>(s.wr) + s.dw, s.r);
+        const V3<T> vo = other(v), co = other(c);
+        return ((second ? vo - v : v - vo) + (second ? co : c)) - (second ? c : co);
+    }
+    __device__ __forceinline__ V3<T> through(const V3<T> &p) const {
+        const V3<T> e = body ? s.through(p) : v3(T(0), T(0), T(0));
+        return e + other(e);
+    }
+    __device__ __forceinline__ V3<T> add_through(const V3<T> &p, const V3<T> *g) const {
+        const V3<T> e = body ? s.through(p) : v3(T(0), T(0), T(0));
+        const V3<T> f = other(e);
+        return (*g + (second ? f : e)) + (second ? e : f);
+    }
+    // the old impulse's corrections, before the current ones are known
+    __device__ __forceinline__ void prepare(const V3<T> &p) {
+        const V3<T> v = s.vr.w * p, w = s.I(cross(s.r, p));
+        ov = second ? v : -v;
+        ow = second ? w : -w;
+    }
+    __device__ __forceinline__ void remove(const V3<T> &) {
+        if (body) {
+            s.dv = s.dv + ov;
+            s.dw = s.dw + ow;
+        }
+    }
+    __device__ __forceinline__ void apply(const V3<T> &p) {
+        const V3<T> v = s.vr.w * p, w = s.I(cross(s.r, p));
+        if (body) {
+            s.dv = s.dv + (second ? -v : v);
+            s.dw = s.dw + (second ? -w : w);
+        }
+    }
+};
+
+// What an update needs of the contact's old impulse pc (contact frame) alone, so that a caller
+// that waits for the bodies' corrections has it before they come.
+template <typename T>
+struct OldImpulse {
+    V3<T> p;   // world frame
+    T en;      // model 1: n . (its tangential part through the bodies' rotations)
+};
+template <typename T, int MODEL, typename S>
+__device__ __forceinline__ OldImpulse<T> relax_old(const T4<T> *R, V3<T> pc, const S &sides) {
+    OldImpulse<T> f;
+    const V3<T> n = xyz<T>(R[0]);
+    f.en = T(0);
+    if (MODEL != 0) {
+        const V3<T> t = xyz<T>(R[3]), o = xyz<T>(R[4]);
+        f.p = n * pc.x + t * pc.y + o * pc.z;
+        if (MODEL == 1) f.en = dot(n, sides.through(t * pc.y + o * pc.z));
+    } else {
+        f.p = n * pc.x;
+    }
+    return f;
+}
+
+// The update of one contact of relaxation model MODEL (pe's RelaxationModel, HCSITS.h:172-179):
+// R its solver record (R[1].w and R[2].w: 1/D_nn and D_nn), push its penetration term distance /
+// dt, dck its Delassus block (models 2-5).  The sides' corrections are updated in place; pcf
+// receives the new impulse in the contact frame, the result is the change of the impulse.
+template <typename T, int MODEL, typename S>
+__device__ __forceinline__ V3<T> relax_contact(const T4<T> *R, T push, const T4<T> *dck, V3<T> pc,
+                                               const OldImpulse<T> &old, S &sides, V3<T> &pcf) {
+    constexpr bool FRICTION = MODEL != 0;
+    const V3<T> n = xyz<T>(R[0]);
+    const T dn_inv = R[1].w;
     V3<T> t, o;
-    V3<T> pold;
     T4<T> q3, q4;
     if (FRICTION) {
         q3 = R[3];
         q4 = R[4];
         t = xyz<T>(q3);
         o = xyz<T>(q4);
-        pold = n * pc.x + t * pc.y + o * pc.z;
-    } else {
-        pold = n * pc.x;
     }
     // remove this contact's impulse (HCSITS.h:2050-2053)
-    dv1 = dv1 - im1 * pold;
-    dw1 = dw1 - I1(cross(r1, pold));
-    if (b2 >= 0) {
-        dv2 = dv2 + im2 * pold;
-        dw2 = dw2 + I2(cross(r2, pold));
-    }
-    const V3<T> gdot = ((v1 + dv1) - (v2 + dv2) + cross(w1 + dw1, r1)) - cross(w2 + dw2, r2);
-    T gn = dot(n, gdot) + dist * dtinv;
+    sides.remove(old.p);
+    const V3<T> gdot = sides.velocity();
+    const T gn = dot(n, gdot) + push;
     V3<T> pnew = v3(T(0), T(0), T(0));
-    V3<T> pcf = pnew;
+    pcf = pnew;
     bool apply = false;
     if (MODEL == 0 || MODEL == 1) {
         if (gn < T(0)) {
@@ -1052,16 +1171,11 @@ __device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
                 T fsq = pcf.y * pcf.y + pcf.z * pcf.z;
                 if (fsq > flimit * flimit || pcf.x < T(0)) {
                     // decoupled relaxation (HCSITS.h:2187-2228)
-                    V3<T> ptmp = t * pc.y + o * pc.z;
-                    const V3<T> e1 = cross(I1(cross(r1, ptmp)), r1);
-                    const V3<T> e2 = (b2 >= 0) ? cross(I2(cross(r2, ptmp)), r2) : v3(T(0), T(0), T(0));
-                    const T gdot_n = gn + dot(n, e1 + e2);
+                    const T gdot_n = gn + old.en;
                     pcf.x = -(dn_inv * gdot_n);
                     pcf.x = pcf.x > T(0) ? pcf.x : T(0);
-                    ptmp = n * pcf.x;
-                    const V3<T> f1 = cross(I1(cross(r1, ptmp)), r1);
-                    const V3<T> f2 = (b2 >= 0) ? cross(I2(cross(r2, ptmp)), r2) : v3(T(0), T(0), T(0));
-                    const V3<T> gdot2 = (gdot + f1) + f2;
+                    const V3<T> ptmp = n * pcf.x;
+                    const V3<T> gdot2 = sides.add_through(ptmp, &gdot);
                     const T g2t = dot(t, gdot2), g2o = dot(o, gdot2);
                     const T ttt = q4.w, tto = q6.z, too = q6.w;
                     pcf.y = -(ttt * g2t + tto * g2o);
@@ -1080,9 +1194,8 @@ __device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
     } else {
         const T mu = q3.w;
         const V3<T> g = v3(gn, dot(t, gdot), dot(o, gdot));
-        const T4<T> *dck = cc.dc_of(k);
         const T4<T> d0 = dck[0], d1 = dck[1];
-        const T D[6] = {q2.w, d0.x, d0.y, d0.z, d0.w, d1.x};   // xx xy xz yy yz zz
+        const T D[6] = {R[2].w, d0.x, d0.y, d0.z, d0.w, d1.x};   // xx xy xz yy yz zz
         if (MODEL == 2 || MODEL == 4) {
             pcf = solve_orthogonal<T, MODEL == 4>(pc, g, D, mu);
             apply = true;
@@ -1095,12 +1208,8 @@ __device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
             const T fsq = pcf.y * pcf.y + pcf.z * pcf.z;
             if (fsq > flimit * flimit || pcf.x < T(0)) {
                 if (MODEL == 3) {
-                    auto corr = [&](const V3<T> &pp) {
-                        const V3<T> e1 = cross(I1(cross(r1, pp)), r1);
-                        const V3<T> e2 = (b2 >= 0) ? cross(I2(cross(r2, pp)), r2) : v3(T(0), T(0), T(0));
-                        return e1 + e2;
-                    };
-                    pcf = solve_coulomb_decoupling<T>(pcf, gdot, n, t, o, dist * dtinv, dn_inv, q4.w,
+                    auto corr = [&](const V3<T> &pp) { return sides.through(pp); };
+                    pcf = solve_coulomb_decoupling<T>(pcf, gdot, n, t, o, push, dn_inv, q4.w,
                                                       q6.z, q6.w, D, mu, corr);
                 } else {
                     pcf = solve_gmd<T>(pcf, g, D, mu, fsq);
@@ -1109,26 +1218,57 @@ __device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
         }
         if (apply) pnew = n * pcf.x + t * pcf.y + o * pcf.z;
     }
-    if (apply) {
-        dv1 = dv1 + im1 * pnew;
-        dw1 = dw1 + I1(cross(r1, pnew));
-        if (b2 >= 0) {
-            dv2 = dv2 - im2 * pnew;
-            dw2 = dw2 - I2(cross(r2, pnew));
-        }
-    }
-    cc.put_p(k, mk4<T>(pcf.x, pcf.y, pcf.z, T(0)));
-    bv.put_dv(b1, mk4<T>(dv1.x, dv1.y, dv1.z, T(0)));
-    bv.put_dw(b1, mk4<T>(dw1.x, dw1.y, dw1.z, T(0)));
+    if (apply) sides.apply(pnew);
+    return old.p - pnew;
+}
+
+template <typename T>
+__device__ __forceinline__ void track_change(const V3<T> &dp, unsigned long long *delta) {
+    const double m = fmax(fabs(double(dp.x)), fmax(fabs(double(dp.y)), fabs(double(dp.z))));
+    atomicMax(delta, (unsigned long long)__double_as_longlong(m));
+}
+
+// one contact of one sweep; COHERENT: read the velocity corrections and the impulse from L2
+template <typename T, int MODEL, bool COHERENT, bool GEN = false, typename BV = BodyV<T>,
+          typename CC = Cache<T>>
+__device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
+                                              const BV &bv, int track_delta,
+                                              unsigned long long *delta) {
+    const int2 ids = cc.get_ids(k);
+    const int32_t b1 = ids.x, b2 = ids.y;
+    const T4<T> *R = cc.rec_of(k);
+    const V3<T> pc = xyz<T>(cc.template get_p<COHERENT>(k));
+    const T4<T> zero = mk4<T>(T(0), T(0), T(0), T(0));
+    BothSides<T, GEN> x;
+    x.two = b2 >= 0;
+    x.a.vr = bv.get_vr(b1);
+    x.a.wr = bv.get_wr(b1);
+    x.a.dv = xyz<T>(bv.template get_dv<COHERENT>(b1));
+    x.a.dw = xyz<T>(bv.template get_dw<COHERENT>(b1));
+    x.b.vr = x.b.wr = zero;
+    x.b.dv = x.b.dw = xyz<T>(zero);
     if (b2 >= 0) {
-        bv.put_dv(b2, mk4<T>(dv2.x, dv2.y, dv2.z, T(0)));
-        bv.put_dw(b2, mk4<T>(dw2.x, dw2.y, dw2.z, T(0)));
+        x.b.vr = bv.get_vr(b2);
+        x.b.wr = bv.get_wr(b2);
+        x.b.dv = xyz<T>(bv.template get_dv<COHERENT>(b2));
+        x.b.dw = xyz<T>(bv.template get_dw<COHERENT>(b2));
     }
-    if (track_delta) {
-        const V3<T> dp = pold - pnew;
-        const double m = fmax(fabs(double(dp.x)), fmax(fabs(double(dp.y)), fabs(double(dp.z))));
-        atomicMax(delta, (unsigned long long)__double_as_longlong(m));
+    x.a.r = xyz<T>(R[1]);
+    x.b.r = xyz<T>(R[2]);
+    x.a.I = load_invi<T, GEN>(bv, b1, x.a.wr.w);
+    x.b.I = load_invi<T, GEN>(bv, b2, x.b.wr.w);
+    static_assert(!GEN || std::is_same<BV, BodyV<T>>::value, "full inverse inertias: BodyV only");
+    V3<T> pcf;
+    const OldImpulse<T> old = relax_old<T, MODEL>(R, pc, x);
+    const V3<T> dp = relax_contact<T, MODEL>(R, R[0].w * dtinv, cc.dc_of(k), pc, old, x, pcf);
+    cc.put_p(k, mk4<T>(pcf.x, pcf.y, pcf.z, T(0)));
+    bv.put_dv(b1, mk4<T>(x.a.dv.x, x.a.dv.y, x.a.dv.z, T(0)));
+    bv.put_dw(b1, mk4<T>(x.a.dw.x, x.a.dw.y, x.a.dw.z, T(0)));
+    if (b2 >= 0) {
+        bv.put_dv(b2, mk4<T>(x.b.dv.x, x.b.dv.y, x.b.dv.z, T(0)));
+        bv.put_dw(b2, mk4<T>(x.b.dw.x, x.b.dw.y, x.b.dw.z, T(0)));
     }
+    if (track_delta) track_change<T>(dp, delta);
 }
 
 // Whether a sweep form runs for this step (decided on the device, so that a step can be queued
@@ -1137,7 +1277,8 @@ __device__ __forceinline__ void sweep_contact(int64_t k, T dtinv, const CC &cc,
 // Gates 4 and 5 split gate 1 by the contact count: 4 when the compact single-block form holds
 // them all (kCompactMax), 5 when it does not.  Gate 3 (the cluster form) runs for colours beyond
 // one block up to kDsmemMaxcol, and gate 6 (the grid, when the cluster form is launched beside
-// it) for larger ones.
+// it) for larger ones.  Gates 7 and 8 split the steps by the contact count alone: 8 (the compact
+// form beside the form without barriers) up to kCompactMax contacts, 7 (the latter) beyond.
 constexpr int kCompactMax = 768;      // contacts of the compact single-block form
 constexpr int kDsmemMaxcol = 3072;    // largest colour the cluster form takes in automatic mode
 __device__ __forceinline__ bool sweeps_gate(const int32_t *dd, int gate) {
@@ -1147,6 +1288,8 @@ __device__ __forceinline__ bool sweeps_gate(const int32_t *dd, int gate) {
     if ((gate == 1 || gate == 4 || gate == 5) && maxcol > kBlk) return false;
     if (gate == 4 && nc > kCompactMax) return false;
     if (gate == 5 && nc <= kCompactMax) return false;
+    if (gate == 7 && nc <= kCompactMax) return false;
+    if (gate == 8 && nc > kCompactMax) return false;
     if ((gate == 2 || gate == 3 || gate == 6) && maxcol <= kBlk) return false;
     if (gate == 3 && maxcol > kDsmemMaxcol) return false;
     if (gate == 6 && maxcol <= kDsmemMaxcol) return false;
@@ -1551,6 +1694,224 @@ __global__ void __launch_bounds__(kDsBlk) k_sweeps_dsmem(int iters, const int32_
     }
 }
 
+// ---- sweeps without barriers ------------------------------------------------------------------
+// All sweeps of a step in one cooperative launch with no barrier between the colours: a warp
+// owns its contacts for all sweeps, and a contact's update waits only for its two bodies.  With
+// colours taken in order a body's d contacts update it in a fixed cycle; each hands the body's
+// corrections to the next one, by storing them into that contact's mailbox (one per side) as
+// 16-byte vectors that each carry a tag: it + 1 from an update in sweep it.  A contact that is
+// its body's first waits for tag it (zeroed mailboxes: no correction before sweep 0), another for
+// it + 1; a contact that has its body to itself keeps the corrections in registers.  The next
+// store into a mailbox comes after the cycle has passed through its reader, so one is enough.  The
+// vectors are single 128-bit relaxed accesses in L2, so no fence orders them.  Per body, the
+// updates come in exactly the colour order of the other forms: the results are the same bits.
+//   Progress: a warp takes groups of contacts of one colour in (sweep, colour) order, its lanes
+// together (they share no body), and all blocks are resident (cooperative launch), so the least
+// unfinished group is always some warp's current one.  Polls are bounded: a warp that gives up
+// raises DERR_TIMEOUT, which ends the others.
+//   Bound: the chain of updates on a body, which takes at most one step per colour: the update
+// itself (700 cycles in FP64 without friction, 1100 in FP32 with it), its store into the L2 and the
+// poll that sees it (a lone store and poll take 470 cycles within a die and 850 across, a poll of
+// a warp's mailboxes about 900).  100 sweeps of 8 colours: 1.26 ms in FP32 with friction (50,000
+// contacts, 2.2 ms with staged records and a grid barrier) and 1.28 ms in FP64 without (32,000
+// contacts, 3.0 ms in one cluster's shared memory); 39 colours of a box stack: 5.5 ms against 7.3
+// in one block.  Polling through one small tag per mailbox before loading it was slower (1.63 and
+// 1.49 ms): the traffic of the polls is not what bounds it.
+template <typename T> struct FlowRec;
+template <>
+struct FlowRec<float> {
+    static constexpr int N = 2;   // [dv, version] [dw, version]
+    static __device__ __forceinline__ bool unpack(const ulonglong2 *q, uint32_t ver, V3<float> &dv,
+                                                  V3<float> &dw) {
+        dv = v3(__uint_as_float((uint32_t)q[0].x), __uint_as_float((uint32_t)(q[0].x >> 32)),
+                __uint_as_float((uint32_t)q[0].y));
+        dw = v3(__uint_as_float((uint32_t)q[1].x), __uint_as_float((uint32_t)(q[1].x >> 32)),
+                __uint_as_float((uint32_t)q[1].y));
+        return (uint32_t)(q[0].y >> 32) == ver && (uint32_t)(q[1].y >> 32) == ver;
+    }
+    static __device__ __forceinline__ void pack(ulonglong2 *q, uint32_t ver, const V3<float> &dv,
+                                                const V3<float> &dw) {
+        auto two = [](uint32_t lo, uint32_t hi) { return (unsigned long long)lo | ((unsigned long long)hi << 32); };
+        q[0] = make_ulonglong2(two(__float_as_uint(dv.x), __float_as_uint(dv.y)), two(__float_as_uint(dv.z), ver));
+        q[1] = make_ulonglong2(two(__float_as_uint(dw.x), __float_as_uint(dw.y)), two(__float_as_uint(dw.z), ver));
+    }
+};
+template <>
+struct FlowRec<double> {
+    static constexpr int N = 4;   // twelve 32-bit words of dv, dw, three and the version per vector
+    static __device__ __forceinline__ bool unpack(const ulonglong2 *q, uint32_t ver, V3<double> &dv,
+                                                  V3<double> &dw) {
+        uint32_t w[12];
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            w[3 * k] = (uint32_t)q[k].x;
+            w[3 * k + 1] = (uint32_t)(q[k].x >> 32);
+            w[3 * k + 2] = (uint32_t)q[k].y;
+            ok = ok && (uint32_t)(q[k].y >> 32) == ver;
+        }
+        auto d = [&](int i) { return __hiloint2double((int)w[2 * i + 1], (int)w[2 * i]); };
+        dv = v3(d(0), d(1), d(2));
+        dw = v3(d(3), d(4), d(5));
+        return ok;
+    }
+    static __device__ __forceinline__ void pack(ulonglong2 *q, uint32_t ver, const V3<double> &dv,
+                                                const V3<double> &dw) {
+        const double x[6] = {dv.x, dv.y, dv.z, dw.x, dw.y, dw.z};
+        uint32_t w[12];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            w[2 * i] = (uint32_t)__double2loint(x[i]);
+            w[2 * i + 1] = (uint32_t)__double2hiint(x[i]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            q[k] = make_ulonglong2((unsigned long long)w[3 * k] | ((unsigned long long)w[3 * k + 1] << 32),
+                                   (unsigned long long)w[3 * k + 2] | ((unsigned long long)ver << 32));
+    }
+};
+
+__device__ __forceinline__ ulonglong2 ld_flow(const ulonglong2 *p) {
+    ulonglong2 r;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+                 : "=l"(r.x), "=l"(r.y) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ void st_flow(ulonglong2 *p, const ulonglong2 &v) {
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+                 :: "l"(p), "l"(v.x), "l"(v.y) : "memory");
+}
+
+constexpr int kFlowBlk = 128;
+
+// Two lanes share a contact, one for each of its bodies.  cc.mail: the mailboxes, vector q of side
+// s of contact k at 2 (q cap + k) + s, zeroed; cc.seq: per contact, the place among its bodies'
+// contacts and their number {s1, d1, s2, d2}; adj: every body's contacts in colour order
+// (2 k + side), body b's from adj_start[b].
+template <typename T, int MODEL, bool GEN>
+__global__ void __launch_bounds__(kFlowBlk, sizeof(T) == 4 ? 5 : 3)
+    k_sweeps_flow(int iters, const int32_t *dd, int gate, const int32_t *color_start, int64_t cap,
+                  T dtinv, Cache<T> cc, BodyV<T> bv, const int32_t *adj_start, const int32_t *adj,
+                  int track_last, unsigned long long *delta, int32_t *err) {
+    constexpr int N = FlowRec<T>::N;
+    if (!sweeps_gate(dd, gate)) return;
+    if (*(volatile int32_t *)err & DERR_COLORS) return;   // no valid colouring to follow
+    __shared__ int32_t cs[kMaxColors + 1], goff[kMaxColors + 1];
+    __shared__ int s_size;
+    const int ncolors = dd[kDdNcolors];
+    const int warps = (int)gridDim.x * (kFlowBlk / 32);
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i <= ncolors; i += kFlowBlk) cs[i] = color_start[i];
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        // groups of `size` contacts of one colour: the smallest with a warp for every group
+        auto groups = [&](int size) {
+            int g = 0;
+            for (int c = lane; c < ncolors; c += 32) g += (cs[c + 1] - cs[c] + size - 1) / size;
+            return __reduce_add_sync(0xffffffffu, g);
+        };
+        int size = min(16, max(1, (cs[ncolors] + warps - 1) / warps));
+        while (size < 16 && groups(size) > warps) ++size;
+        if (lane == 0) {
+            int off = 0;
+            for (int c = 0; c < ncolors; ++c) {
+                goff[c] = off;
+                off += (cs[c + 1] - cs[c] + size - 1) / size;
+            }
+            goff[ncolors] = off;
+            s_size = size;
+        }
+    }
+    __syncthreads();
+    const int size = s_size, ngroups = goff[ncolors];
+    // neighbouring groups on different SMs
+    const int warp = (int)blockIdx.x + (int)gridDim.x * (int)(threadIdx.x >> 5);
+    const bool single = warp + warps >= ngroups;   // the warp keeps one group in registers
+    int loaded = -1, col = 0;
+    // the lane's contact of the current group: its record and this lane's body
+    int k = 0;
+    bool live = false;
+    int32_t b = -1;
+    int place = 0, count = 0;
+    T4<T> R[kRec];
+    PairedSides<T, GEN> x;
+    x.second = (lane & 1) != 0;
+    V3<T> pc;
+    int32_t from = 0, to = 0;   // its mailbox, and that of its body's next contact
+    for (int it = 0; it < iters; ++it) {
+        for (int g = warp; g < ngroups; g += warps) {
+            if (g != loaded) {
+                __syncwarp();   // a pair's impulse is stored by one lane and read by both
+                if (g < loaded) col = 0;
+                loaded = g;
+                while (g >= goff[col + 1]) ++col;
+                k = cs[col] + (g - goff[col]) * size + (lane >> 1);
+                live = lane < 2 * size && k < cs[col + 1];
+                if (!live) k = cs[col];   // an idle pair takes a valid contact and waits for nothing
+                const int2 ids = cc.ids[k];
+                const int4 sq = cc.seq[k];
+                b = x.second ? ids.y : ids.x;
+                place = x.second ? sq.z : sq.x;
+                count = x.second ? sq.w : sq.y;
+                x.body = b >= 0;
+                const T4<T> *r = cc.rec + (int64_t)kRec * k;
+#pragma unroll
+                for (int q = 0; q < (MODEL == 0 ? 3 : kRec); ++q) R[q] = r[q];
+                x.s.r = x.second ? xyz<T>(R[2]) : xyz<T>(R[1]);
+                pc = xyz<T>(cc.p[k]);
+                x.s.vr = x.s.wr = mk4<T>(T(0), T(0), T(0), T(0));
+                x.s.dv = x.s.dw = v3(T(0), T(0), T(0));
+                if (x.body) {
+                    x.s.vr = bv.vr[b];
+                    x.s.wr = bv.wr[b];
+                }
+                x.s.I = load_invi<T, GEN>(bv, b, x.s.wr.w);
+                from = 2 * k + (x.second ? 1 : 0);
+                if (live && x.body) to = adj[adj_start[b] + (place + 1 == count ? 0 : place + 1)];
+            }
+            // alone on a body, with the group in registers: nothing to wait for after sweep 0
+            const bool own = single && count == 1;
+            const uint32_t tag = (uint32_t)it + (place > 0 ? 1u : 0u);
+            bool need = live && x.body && !(own && it > 0);
+            const OldImpulse<T> old = relax_old<T, MODEL>(R, pc, x);
+            x.prepare(old.p);
+            const T push = R[0].w * dtinv;
+            ulonglong2 q4[N];
+            // the contacts of a group share no body, so its lanes wait together
+            for (unsigned int spins = 0;;) {
+                if (need) {
+#pragma unroll
+                    for (int q = 0; q < N; ++q) q4[q] = ld_flow(cc.mail + from + 2 * q * cap);
+                    need = !FlowRec<T>::unpack(q4, tag, x.s.dv, x.s.dw);
+                }
+                if (!__any_sync(0xffffffffu, need)) break;
+                if (((++spins) & 0xfffu) == 0u) {
+                    if (spins > (unsigned int)kSpinLimit) atomicOr(err, DERR_TIMEOUT);
+                    if (__any_sync(0xffffffffu, (*(volatile int32_t *)err & DERR_TIMEOUT) != 0)) return;
+                }
+            }
+            V3<T> pcf;
+            const V3<T> dp = relax_contact<T, MODEL>(R, push, cc.dc_of(k), pc, old, x, pcf);
+            if (live && x.body && !own) {
+                FlowRec<T>::pack(q4, (uint32_t)it + 1u, x.s.dv, x.s.dw);
+#pragma unroll
+                for (int q = 0; q < N; ++q) st_flow(cc.mail + to + 2 * q * cap, q4[q]);
+            }
+            pc = pcf;
+            if (live && !x.second && (it == iters - 1 || !single))
+                cc.p[k] = mk4<T>(pcf.x, pcf.y, pcf.z, T(0));
+            if (live && it == iters - 1) {
+                // the last update of a body leaves its corrections for the integration
+                if (x.body && place == count - 1) {
+                    bv.put_dv(b, mk4<T>(x.s.dv.x, x.s.dv.y, x.s.dv.z, T(0)));
+                    bv.put_dw(b, mk4<T>(x.s.dw.x, x.s.dw.y, x.s.dw.z, T(0)));
+                }
+                if (track_last && !x.second) track_change<T>(dp, delta);
+            }
+        }
+    }
+}
+
 // complementarity residual of the final impulses (same definition as the oracle), in FP64
 template <typename T, bool FRICTION>
 __global__ void k_residual(const int32_t *ncp, int64_t cap, double dtinv, Cache<T> cc,
@@ -1676,8 +2037,8 @@ int nbgs_alloc(Ctx *c, int64_t cap) {
         b.color = nullptr;
         dfree(c, b.body_adj);
         b.body_adj = nullptr;
-        // raw: 2 int + 11 T; cache: 2 int + (kRec + 3) x 4 T  (per contact)
-        const size_t bytes = (size_t)cap * (4 * sizeof(int32_t) + (11 + 4 * (kRec + 3)) * es) + 64 * 256;
+        // raw: 2 int + 11 T; cache: 6 int + (kRec + 3) x 4 T, and 16 T of mailboxes (per contact)
+        const size_t bytes = (size_t)cap * (8 * sizeof(int32_t) + (11 + 4 * (kRec + 3) + 16) * es) + 64 * 256;
         PEB_CUDA(c, dmalloc(c, &b.cache, bytes));
         PEB_CUDA(c, dmalloc(c, &b.order, (size_t)cap * sizeof(int32_t)));
         PEB_CUDA(c, dmalloc(c, &b.color, (size_t)cap * sizeof(int32_t)));
@@ -1760,6 +2121,8 @@ void layout(Ctx *c, Raw<T> &raw, Cache<T> &cc, BodyV<T> &bv) {
     cc.rec = (T4<T> *)take(kRec * cap * sizeof(T4<T>));
     cc.p = (T4<T> *)take(cap * sizeof(T4<T>));
     cc.dc = (T4<T> *)take(2 * cap * sizeof(T4<T>));
+    cc.seq = (int4 *)take(cap * sizeof(int4));
+    cc.mail = (ulonglong2 *)take(cap * 16 * sizeof(T));
     const int64_t n = b.nbod;
     T4<T> *v = (T4<T> *)b.vel;
     bv.vr = v;
@@ -2123,6 +2486,66 @@ int launch_sweeps_dsmem(Ctx *c, int model, int iters, int gate, int64_t cap, VT 
     return PE_B200_OK;
 }
 
+template <typename VT, bool GEN>
+auto flow_kernel_g(int m) -> decltype(&k_sweeps_flow<VT, 0, GEN>) {
+    switch (m) {
+        case 1: return k_sweeps_flow<VT, 1, GEN>;
+        case 2: return k_sweeps_flow<VT, 2, GEN>;
+        case 3: return k_sweeps_flow<VT, 3, GEN>;
+        case 4: return k_sweeps_flow<VT, 4, GEN>;
+        case 5: return k_sweeps_flow<VT, 5, GEN>;
+        default: return k_sweeps_flow<VT, 0, GEN>;
+    }
+}
+template <typename VT>
+auto flow_kernel(int m, bool gen) -> decltype(&k_sweeps_flow<VT, 0, false>) {
+    if constexpr (std::is_same<VT, double>::value) {
+        if (gen) return flow_kernel_g<VT, true>(m);
+    }
+    return flow_kernel_g<VT, false>(m);
+}
+
+// Launches k_sweeps_flow: as many blocks as are resident together, six per SM at most (a warp
+// then holds a few contacts; more warps only add polls); *done reports it.
+template <typename VT>
+int launch_sweeps_flow(Ctx *c, int model, bool gen, int iters, int gate, int64_t cap, VT dtinv,
+                       const Cache<VT> &cc, const BodyV<VT> &bv, int track,
+                       unsigned long long *dl, bool *done) {
+    NbgsBuf &nb = c->nb;
+    *done = false;
+    if (nb.flow_off) return PE_B200_OK;
+    auto kern = flow_kernel<VT>(model, gen);
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kFlowBlk, 0) != cudaSuccess || occ < 1) {
+        cudaGetLastError();
+        nb.flow_off = true;
+        return PE_B200_OK;
+    }
+    constexpr int per_block = kFlowBlk / 32;   // a block per four contacts is the most that helps
+    const int64_t g = std::max<int64_t>(
+        1, std::min<int64_t>((int64_t)std::min(occ, 6) * c->sm_count, (cap + per_block - 1) / per_block));
+    int iters_a = iters, gate_a = gate, track_a = track;
+    int64_t cap_a = cap;
+    VT dtinv_a = dtinv;
+    const int32_t *dd = nb.dd;
+    Cache<VT> cc_a = cc;
+    BodyV<VT> bv_a = bv;
+    const int32_t *adj_start = nb.body_cnt, *adj = nb.body_adj;
+    const int32_t *cs = nb.cstart_dev;
+    void *args[] = {&iters_a, &dd, &gate_a, &cs, &cap_a, &dtinv_a, &cc_a, &bv_a, &adj_start, &adj,
+                    &track_a, &dl, &c->d_err};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kern, dim3((unsigned)g),
+                                                      dim3(kFlowBlk), args, 0, c->stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        nb.flow_off = true;
+        return PE_B200_OK;
+    }
+    c->launches++;
+    *done = true;
+    return PE_B200_OK;
+}
+
 // The colouring rounds of a queued step in one cooperative launch (k_color_rounds); a grid of
 // as many blocks as fit, at most one thread per contact of the capacity.
 template <typename VT>
@@ -2171,6 +2594,20 @@ int launch_sweeps_queued(Ctx *c, int model, bool gen, int iters, int64_t cap, VT
     NbgsBuf &nb = c->nb;
     int32_t *dd = nb.dd;
     const int mode = c->tune.nbgs_sweeps;
+    if (mode == 0 && !gen) {
+        // a few contacts: the compact form; more: the form without barriers
+        bool done = false;
+        int rc = launch_sweeps_flow<VT>(c, model, gen, iters, 7, cap, dtinv, cc, bv, 0, dl, &done);
+        if (rc) return rc;
+        if (done) {
+            rc = launch_sweeps_compact<VT>(c, model, iters, 8, dtinv, cc, bv, 0, dl, &done);
+            if (rc || done) return rc;
+            block_kernel<VT>(model, gen)<<<1, kBlk, 0, c->stream>>>(iters, dd, 8, nb.cstart_dev, cap,
+                                                                    dtinv, cc, bv, n, 0, dl);
+            PEB_LAUNCHED(c);
+            return PE_B200_OK;
+        }
+    }
     // every colour within one block: the compact form for a few contacts, else the whole-scene
     // single-block form
     bool compact = false;
@@ -2386,6 +2823,10 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     // 3. colouring
     int32_t ncolors = 0;
     const bool any = queued ? !nb.plan_none : nc > 0;
+    // the sweeps without barriers may run: k_cache writes the bodies' contacts in colour order
+    // (over the colouring's adjacency, which it no longer needs)
+    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && (queued || gen || nc > kCompactMax)
+                            ? nb.body_adj : nullptr;
     if (any) {
         prof_begin(c, ST_COLOR);
         const size_t masks = (size_t)nbod * (gen ? 4 : 1) * sizeof(uint64_t);
@@ -2394,18 +2835,20 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         // the body -> contacts adjacency of the parallel rounds (skipped on the device, or by the
         // host, when one thread colours the step)
         const int32_t *rounds = queued ? dd + kDdRounds : nullptr;
-        if (queued || nc > serial_max) {
+        if (queued || nc > serial_max || flow_adj) {
             PEB_CUDA(c, cudaMemsetAsync(nb.body_cnt, 0, ((size_t)nbod + 1) * sizeof(int32_t), c->stream));
             k_degree<<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, rounds, raw.b1, raw.b2, nb.body_cnt);
             PEB_LAUNCHED(c);
             rc = scan_exclusive_cond(c, nb.body_cnt, nb.body_cnt, nbod, rounds);
             if (rc) return rc;
-            int32_t *fill = nb.cnt;  // reuse: counts are consumed
-            PEB_CUDA(c, cudaMemcpyAsync(fill, nb.body_cnt, ((size_t)nbod + 1) * sizeof(int32_t),
-                                        cudaMemcpyDeviceToDevice, c->stream));
-            k_adj_fill<<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, rounds, raw.b1, raw.b2, fill,
-                                                      nb.body_adj);
-            PEB_LAUNCHED(c);
+            if (queued || nc > serial_max) {
+                int32_t *fill = nb.cnt;  // reuse: counts are consumed
+                PEB_CUDA(c, cudaMemcpyAsync(fill, nb.body_cnt, ((size_t)nbod + 1) * sizeof(int32_t),
+                                            cudaMemcpyDeviceToDevice, c->stream));
+                k_adj_fill<<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, rounds, raw.b1, raw.b2, fill,
+                                                          nb.body_adj);
+                PEB_LAUNCHED(c);
+            }
         }
         PEB_CUDA(c, cudaMemsetAsync(nb.color, 0xff, (size_t)(queued ? cap : nc) * sizeof(int32_t), c->stream));
         const int words = gen ? 4 : 1;
@@ -2413,7 +2856,7 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         if (queued) {
             // one thread for a few contacts; otherwise every round in one cooperative launch
             k_color_serial<1><<<1, 256, in_smem ? masks : 0, c->stream>>>(
-                ncp, dd, serial_max, raw.b1, raw.b2, nb.color, nbod, in_smem ? nullptr : nb.used,
+                ncp, dd, serial_max, raw.b1, raw.b2, nb.color, nbod, nb.used, in_smem ? 1 : 0,
                 c->d_err);
             PEB_LAUNCHED(c);
             PEB_CUDA(c, cudaMemsetAsync(nb.rem, 0, kMaxRounds * sizeof(int32_t), c->stream));
@@ -2423,7 +2866,7 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
             int round = 0;
             if (nc <= serial_max) {
                 (gen ? k_color_serial<4> : k_color_serial<1>)<<<1, 256, in_smem ? masks : 0, c->stream>>>(
-                    ncp, dd, serial_max, raw.b1, raw.b2, nb.color, nbod, in_smem ? nullptr : nb.used,
+                    ncp, dd, serial_max, raw.b1, raw.b2, nb.color, nbod, nb.used, in_smem ? 1 : 0,
                     c->d_err);
                 PEB_LAUNCHED(c);
             }
@@ -2470,10 +2913,10 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         prof_begin(c, ST_CACHE);
         // 4. contact cache in colour-sorted order
         if constexpr (std::is_same<VT, double>::value) {
-            if (gen) k_cache<VT, true><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, bv, n, cc);
-            else k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, bv, n, cc);
+            if (gen) k_cache<VT, true><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
+            else k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
         } else {
-            k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, bv, n, cc);
+            k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
         }
         PEB_LAUNCHED(c);
         prof_end(c, ST_CACHE);
@@ -2513,6 +2956,12 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
             // a few contacts: one block with their bodies in shared memory
             int rc = launch_sweeps_compact<VT>(c, model, iters, 0, VT(1.0 / dt), cc, bv,
                                               c->want_residual ? 1 : 0, dl, &done);
+            if (rc) return rc;
+        }
+        if (!done && mode == 0 && flow_adj) {
+            // the form without barriers
+            int rc = launch_sweeps_flow<VT>(c, model, gen, iters, 0, cap, VT(1.0 / dt), cc, bv,
+                                            c->want_residual ? 1 : 0, dl, &done);
             if (rc) return rc;
         }
         if (!done && mode == 0 && maxcol > kBlk && maxcol <= kDsmemMaxcol) {
