@@ -31,9 +31,9 @@
 #include <math_constants.h>
 
 #include <algorithm>
-#include <climits>
 
 #include "internal.cuh"
+#include "near.cuh"
 #include "rebuild.cuh"
 
 namespace peb {
@@ -594,7 +594,6 @@ __device__ __forceinline__ void grid_forces_sorted(const DemArgs<VT> &a, const S
 // scan visits them (ascending slot), takes each through k_dem_step's exact test and pair force
 // (or, for a sphere with more than kNear, searches its cells again), then the walls and the
 // integration.  Same terms in the same order: bitwise the results of k_dem_step.
-constexpr int kNear = 16;
 constexpr int kNearBlock = 256;
 
 __global__ void __launch_bounds__(kNearBlock, 5) k_grid_near(
@@ -677,29 +676,8 @@ __global__ void __launch_bounds__(kDemBlock) k_dem_near(DemArgs<VT> a,
     if (cnt > kNear) {
         grid_forces_sorted<T, VT, HERTZ>(a, s, posf, t, b, pi, vi, wi, uidi, mi, acc);
     } else if (cnt > 0) {
-        // the recorded slots in ascending order (a sorting network over registers; empty
-        // places hold INT_MAX and sort last)
         int32_t sl[kNear];
-#pragma unroll
-        for (int k = 0; k < kNear; ++k) sl[k] = k < cnt ? near_idx[(int64_t)k * a.n + t] : INT_MAX;
-        if (cnt > 1) {
-#pragma unroll
-            for (int kk = 2; kk <= kNear; kk <<= 1)
-#pragma unroll
-                for (int j = kk >> 1; j > 0; j >>= 1)
-#pragma unroll
-                    for (int i = 0; i < kNear; ++i) {
-                        const int l = i ^ j;
-                        if (l > i) {
-                            const int32_t x = sl[i], y = sl[l];
-                            const bool up = (i & kk) == 0;
-                            if ((x > y) == up) {
-                                sl[i] = y;
-                                sl[l] = x;
-                            }
-                        }
-                    }
-        }
+        load_near(near_idx, a.n, t, cnt, sl);
 #pragma unroll
         for (int k = 0; k < kNear; ++k) {
             if (k >= cnt) break;
@@ -1013,6 +991,16 @@ DemArgs<VT> dem_args(Ctx *c, double dt) {
     return a;
 }
 
+// the candidate lists of the current state (its sort has run)
+int launch_near(Ctx *c) {
+    PEB_CUDA(c, cudaMemsetAsync(c->near, 0, (size_t)c->n * sizeof(int32_t), c->stream));
+    k_grid_near<<<grid_for(c->n, kNearBlock), kNearBlock, 0, c->stream>>>(
+        c->n, c->sorted, c->cur.pr, c->cur.tag, c->d_scenes, c->cell_start, c->posf, c->near,
+        c->near + c->n);
+    PEB_LAUNCHED(c);
+    return PE_B200_OK;
+}
+
 template <typename VT>
 int launch_dem(Ctx *c, double dt) {
     DemArgs<VT> a = dem_args<VT>(c, dt);
@@ -1030,11 +1018,8 @@ int launch_dem(Ctx *c, double dt) {
     } else {
         const float4 *pf = c->posf;
         const int32_t *nc = c->near, *ni = c->near + c->n;
-        PEB_CUDA(c, cudaMemsetAsync(c->near, 0, (size_t)c->n * sizeof(int32_t), c->stream));
-        k_grid_near<<<grid_for(c->n, kNearBlock), kNearBlock, 0, c->stream>>>(
-            c->n, c->sorted, c->cur.pr, c->cur.tag, c->d_scenes, c->cell_start, pf, c->near,
-            c->near + c->n);
-        PEB_LAUNCHED(c);
+        const int rc = launch_near(c);
+        if (rc) return rc;
         if (a.hertz) {
             if (c->p.track_orientation) k_dem_near<VT, true, true><<<g, kDemBlock, 0, c->stream>>>(a, pf, nc, ni);
             else k_dem_near<VT, false, true><<<g, kDemBlock, 0, c->stream>>>(a, pf, nc, ni);
@@ -1443,20 +1428,31 @@ __global__ void k_set_one(int32_t *p) { *p = 1; }
 
 }  // namespace
 
+namespace {
+// the sort of the current state, with the FP32 position copy of the default grid form
+int dem_sort(Ctx *c, bool with_pos) {
+    if (!c->binned) {
+        const int rc = grid_bin_current(c);
+        if (rc) return rc;
+    }
+    if (with_pos && !c->posf) {
+        PEB_CUDA(c, dmalloc(c, &c->posf, (size_t)c->n * sizeof(float4)));
+        PEB_CUDA(c, dmalloc(c, &c->near, (size_t)c->n * (1 + kNear) * sizeof(int32_t)));
+    }
+    return grid_sort(c, with_pos);
+}
+}  // namespace
+
+// the sort and the candidate lists of the current state, without a step
+int dem_search(Ctx *c) {
+    const int rc = dem_sort(c, true);
+    return rc ? rc : launch_near(c);
+}
+
 int dem_step(Ctx *c, double dt) {
     int rc;
     if (c->n > 0) {
-        if (!c->binned) {
-            rc = grid_bin_current(c);
-            if (rc) return rc;
-        }
-        // the sorted FP32 position copy of the default grid form
-        const bool with_pos = c->tune.dem_grid != 1;
-        if (with_pos && !c->posf) {
-            PEB_CUDA(c, dmalloc(c, &c->posf, (size_t)c->n * sizeof(float4)));
-            PEB_CUDA(c, dmalloc(c, &c->near, (size_t)c->n * (1 + kNear) * sizeof(int32_t)));
-        }
-        rc = grid_sort(c, with_pos);
+        rc = dem_sort(c, c->tune.dem_grid != 1);
         if (rc) return rc;
     }
     // moving boxes: their forces on the spheres and their own step, from the current state

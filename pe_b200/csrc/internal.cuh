@@ -199,7 +199,9 @@ struct AdjState {
     int32_t nsteps = 0, every = 1;
     double dt = 0.0;
     std::vector<BodyBuf> ckpt;   // state before steps 0, every, 2*every, ...
-    std::vector<BodyBuf> seg;    // pre-step states of the segment being reversed
+    std::vector<BodyBuf> seg;    // pre-step states of the segment being reversed, after the first
+    int32_t *search = nullptr;   // their sorts and candidate lists, while they are small enough
+    int64_t search_bytes = 0;
 };
 
 // stage timers (pe's profiling sections, e.g. DEMSolver.h:1159-1260): CUDA events around each
@@ -409,6 +411,7 @@ int set_list_skin(Ctx *c, double skin);
 int set_tuning(Ctx *c, const Tuning &t, double skin);
 int autotune(Ctx *c, double dt, int32_t trial, pe_b200_tuning *out);
 int dem_step(Ctx *c, double dt);
+int dem_search(Ctx *c);   // sort and candidate lists of the current state, without a step
 int adjoint_forward(Ctx *c, int32_t nsteps, double dt, int32_t every);
 int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *gw, double *ox,
                      double *ov, double *ow, double *gpar);
