@@ -145,6 +145,7 @@ void free_device(Ctx *c) {
     dfree(c, c->key);
     dfree(c, c->rank);
     dfree(c, c->sorted);
+    dfree(c, c->raw);
     dfree(c, c->cell_count);
     dfree(c, c->cell_start);
     dfree(c, c->scan_tmp);
@@ -163,7 +164,7 @@ void free_device(Ctx *c) {
     dfree(c, c->d_plane_mat);
     dfree(c, c->d_boxes);
     dfree(c, c->d_box_mat);
-    c->key = c->rank = c->sorted = c->cell_count = c->cell_start = c->scan_tmp = nullptr;
+    c->key = c->rank = c->sorted = c->raw = c->cell_count = c->cell_start = c->scan_tmp = nullptr;
     c->scan_tmp_cap = 0;
     c->d_scenes = nullptr;
     c->d_mats = nullptr;

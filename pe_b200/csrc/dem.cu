@@ -1495,7 +1495,7 @@ int dem_list_alloc(Ctx *c) {
             tpsm = 2048;
         }
         const int64_t blk = (int64_t)(tpsm / kRbBlock) * std::max(c->sm_count, 1) + 1;
-        PEB_CUDA(c, dmalloc(c, &L.rb_blk, (size_t)blk * sizeof(int32_t)));
+        PEB_CUDA(c, dmalloc(c, &L.rb_blk, (size_t)blk * sizeof(unsigned long long)));
         L.rb_blk_cap = blk;
     }
     PEB_CUDA(c, dmalloc(c, &L.tmp.pr, n * sizeof(double4)));

@@ -7,8 +7,9 @@
 //   count  (atomic histogram; the producing step kernel already did this for the next step)
 //   scan   (exclusive prefix sum over cells -> cell_start)
 //   scatter(slot of body i = cell_start[key[i]] + rank[i])
-//   fixup  (order each cell by body index, so the result is independent of atomic order)
-// Outside graph captures the three run in one cooperative kernel (k_grid_sort) with bounded grid
+//   order  (each cell by body index, so the result is independent of atomic order; a body finds
+//           its place from the indexes of its cell's bodies)
+// Outside graph captures they run in one cooperative kernel (k_grid_sort) with bounded grid
 // barriers between them, which also clears the counts for the next step; in a capture, and with
 // rebuild_per_sm = -1 (no cooperative launches), they run as separate kernels.  Both give the
 // same arrays.
@@ -104,66 +105,54 @@ __global__ void k_scatter(int64_t n, const int32_t *__restrict__ key,
     sorted[start[key[i]] + rank[i]] = (int32_t)i;
 }
 
-// one cell's insertion sort by body index, and its FP32 position records (posf non-null)
-__device__ __forceinline__ void fixup_cell(int64_t c, const int32_t *start, int32_t *sorted,
-                                           const double4 *pr, const uint32_t *tag,
-                                           const SceneInfo *scenes, float4 *posf) {
-    const int b = start[c], e = start[c + 1];
-    if (e == b) return;
-    for (int i = b + 1; i < e; ++i) {
-        const int32_t v = sorted[i];
-        int j = i - 1;
-        while (j >= b && sorted[j] > v) {
-            sorted[j + 1] = sorted[j];
-            --j;
-        }
-        sorted[j + 1] = v;
-    }
+// body i into its place in cell order, and (posf) its FP32 record: the position relative to its
+// scene's grid origin and the radius (the candidate records of the grid DEM step)
+__device__ __forceinline__ void order_body(int32_t i, const int32_t *__restrict__ raw,
+                                           const int32_t *__restrict__ start,
+                                           const int32_t *__restrict__ key, int32_t *sorted,
+                                           const double4 *__restrict__ pr,
+                                           const uint32_t *__restrict__ tag,
+                                           const SceneInfo *__restrict__ scenes, float4 *posf) {
+    const int32_t t = ordered_slot(raw, start, key[i], i);
+    sorted[t] = i;
     if (!posf) return;
-    for (int i = b; i < e; ++i) {
-        const int32_t j = sorted[i];
-        const double4 p = pr[j];
-        const SceneInfo &s = scenes[tag[j] >> 16];
-        posf[i] = make_float4(float(p.x - s.lo[0]), float(p.y - s.lo[1]), float(p.z - s.lo[2]),
-                              float(p.w));
-    }
+    const double4 p = pr[i];
+    const SceneInfo &s = scenes[tag[i] >> 16];
+    posf[t] = make_float4(float(p.x - s.lo[0]), float(p.y - s.lo[1]), float(p.z - s.lo[2]), float(p.w));
 }
 
-// insertion sort of each cell's slots by body index (cells hold a handful of bodies); with
-// posf, the cell's bodies' positions relative to their scene's grid origin and radii in FP32,
-// in slot order (the candidate records of the grid DEM step)
-__global__ void k_fixup(int64_t ncell, const int32_t *__restrict__ start,
-                        int32_t *__restrict__ sorted, const double4 *__restrict__ pr,
-                        const uint32_t *__restrict__ tag, const SceneInfo *__restrict__ scenes,
-                        float4 *__restrict__ posf) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    fixup_cell(c, start, sorted, pr, tag, scenes, posf);
+__global__ void k_order(int64_t n, const int32_t *__restrict__ raw, const int32_t *__restrict__ start,
+                        const int32_t *__restrict__ key, int32_t *__restrict__ sorted,
+                        const double4 *__restrict__ pr, const uint32_t *__restrict__ tag,
+                        const SceneInfo *__restrict__ scenes, float4 *__restrict__ posf) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) order_body((int32_t)i, raw, start, key, sorted, pr, tag, scenes, posf);
 }
 
 struct GridSortArgs {
     int64_t n, ncell;
-    int32_t *cell_count, *cell_start, *key, *rank, *sorted;
+    int32_t *cell_count, *cell_start, *key, *rank, *raw, *sorted;
     const double4 *pr;
     const uint32_t *tag;
     const SceneInfo *scenes;
     float4 *posf;
     unsigned int *bar;
-    int32_t *blk, *err;
+    unsigned long long *blk;
+    int32_t *err;
 };
 
-// the whole sort in one cooperative grid: scan | scatter, clear the counts | per-cell order
+// the whole sort in one cooperative grid: scan | scatter, clear the counts | order
 __global__ void __launch_bounds__(kRbBlock) k_grid_sort(GridSortArgs g) {
     if (!grid_scan_raw(g.blk, g.bar, g.err, g.cell_count, g.cell_start, g.ncell)) return;
     if (!grid_sync(g.bar, g.err)) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t g0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (int64_t i = g0; i < g.n; i += stride) g.sorted[g.cell_start[g.key[i]] + g.rank[i]] = (int32_t)i;
+    for (int64_t i = g0; i < g.n; i += stride) g.raw[g.cell_start[g.key[i]] + g.rank[i]] = (int32_t)i;
     // the scan has read every count: cleared for the step kernel, which bins for the next sort
     for (int64_t c = g0; c <= g.ncell; c += stride) g.cell_count[c] = 0;
     if (!grid_sync(g.bar, g.err)) return;
-    for (int64_t c = g0; c < g.ncell; c += stride)
-        fixup_cell(c, g.cell_start, g.sorted, g.pr, g.tag, g.scenes, g.posf);
+    for (int64_t i = g0; i < g.n; i += stride)
+        order_body((int32_t)i, g.raw, g.cell_start, g.key, g.sorted, g.pr, g.tag, g.scenes, g.posf);
 }
 
 }  // namespace
@@ -258,7 +247,7 @@ int grid_alloc(Ctx *c) {
             tpsm = 2048;
         }
         c->gs_blk_cap = (int64_t)(tpsm / kRbBlock) * std::max(c->sm_count, 1) + 1;
-        PEB_CUDA(c, dmalloc(c, &c->gs_blk, (size_t)c->gs_blk_cap * sizeof(int32_t)));
+        PEB_CUDA(c, dmalloc(c, &c->gs_blk, (size_t)c->gs_blk_cap * sizeof(unsigned long long)));
     }
     // the scan scratch of every scan a step runs (cells, bodies and moving boxes, list counts),
     // sized here so that no step allocates it inside a graph capture
@@ -267,6 +256,7 @@ int grid_alloc(Ctx *c) {
     PEB_CUDA(c, dmalloc(c, &c->key, n * sizeof(int32_t) + 16));
     PEB_CUDA(c, dmalloc(c, &c->rank, n * sizeof(int32_t) + 16));
     PEB_CUDA(c, dmalloc(c, &c->sorted, n * sizeof(int32_t) + 16));
+    PEB_CUDA(c, dmalloc(c, &c->raw, n * sizeof(int32_t) + 16));
     PEB_CUDA(c, dmalloc(c, &c->cell_count, ((size_t)c->ncell + 1) * sizeof(int32_t)));
     PEB_CUDA(c, dmalloc(c, &c->cell_start, ((size_t)c->ncell + 2) * sizeof(int32_t)));
     return PE_B200_OK;
@@ -307,10 +297,13 @@ int grid_sort(Ctx *c, bool with_pos) {
             c->gs_coop_off = true;
         }
         if (occ > 0) {
-            const int64_t work = std::max<int64_t>(c->ncell, c->n);
+            // a thread per body or per run of the scan; four blocks per SM at most, as many
+            // as their barriers are worth (600,011 spheres, 30 steps and the transfers: 5.61 ms
+            // with four, 5.78 with eight, 5.79 with two, 6.30 with one)
+            const int64_t work = std::max<int64_t>(c->ncell / kScanRun, c->n);
             const int64_t want = std::max<int64_t>(1, (work + kRbBlock - 1) / kRbBlock);
             const unsigned grid = (unsigned)std::min<int64_t>(
-                std::min<int64_t>(want, (int64_t)occ * c->sm_count), c->gs_blk_cap - 1);
+                std::min<int64_t>(want, (int64_t)std::min(occ, 4) * c->sm_count), c->gs_blk_cap - 1);
             GridSortArgs g;
             g.n = c->n;
             g.ncell = c->ncell;
@@ -318,6 +311,7 @@ int grid_sort(Ctx *c, bool with_pos) {
             g.cell_start = c->cell_start;
             g.key = c->key;
             g.rank = c->rank;
+            g.raw = c->raw;
             g.sorted = c->sorted;
             g.pr = c->cur.pr;
             g.tag = c->cur.tag;
@@ -343,10 +337,10 @@ int grid_sort(Ctx *c, bool with_pos) {
     if (rc) return rc;
     if (c->n > 0) {
         k_scatter<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->key, c->rank,
-                                                              c->cell_start, c->sorted);
+                                                              c->cell_start, c->raw);
         PEB_LAUNCHED(c);
-        k_fixup<<<grid_for(c->ncell, 256), 256, 0, c->stream>>>(
-            c->ncell, c->cell_start, c->sorted, c->cur.pr, c->cur.tag, c->d_scenes,
+        k_order<<<grid_for(c->n, 256), 256, 0, c->stream>>>(
+            c->n, c->raw, c->cell_start, c->key, c->sorted, c->cur.pr, c->cur.tag, c->d_scenes,
             with_pos ? c->posf : nullptr);
         PEB_LAUNCHED(c);
     }

@@ -163,7 +163,7 @@ struct ListBuf {
     void *facc = nullptr;
     // persistent rebuild kernel (rebuild.cu): grid barrier words and per-block partial sums
     unsigned int *rb_bar = nullptr;
-    int32_t *rb_blk = nullptr;
+    unsigned long long *rb_blk = nullptr;
     int64_t rb_blk_cap = 0;
     bool coop_disabled = false;
     bool fuse_off = false;   // the fused rebuild-and-contacts kernel cannot be launched here
@@ -253,13 +253,14 @@ struct Ctx {
     int64_t ncell = 0;              // total cells over scenes
     BodyBuf cur, nxt;
     int32_t *key = nullptr, *rank = nullptr, *sorted = nullptr;
+    int32_t *raw = nullptr;         // the sort's scatter, before each cell is put in body order
     int32_t *cell_count = nullptr, *cell_start = nullptr;
     int32_t *scan_tmp = nullptr;
     int64_t scan_tmp_cap = 0;
     // the one-kernel grid sort (grid.cu): barrier counters, per-block partial sums for the
     // largest resident grid, and whether cooperative launches were refused here
     unsigned int *gs_bar = nullptr;
-    int32_t *gs_blk = nullptr;
+    unsigned long long *gs_blk = nullptr;
     int64_t gs_blk_cap = 0;
     bool gs_coop_off = false;
     float4 *posf = nullptr;         // grid step: FP32 positions relative to the grid origin and

@@ -2,10 +2,10 @@
 // of a cooperative grid with bounded grid barriers between them (rebuild.cu's k_rebuild, and the
 // rebuild-and-contacts kernel of the list step in dem.cu):
 //   clear cell counts | bin (cell key + slot, atomic histogram) | scan counts -> cell offsets |
-//   scatter | order each cell by body index | gather bodies into cell order (the list buffers'
-//   copy of the state, which the force kernels of the step read instead of the current one) |
-//   count neighbours closer than r_i + r_j + skin (keeping the first few), mark the spheres that
-//   can feel a force before the next rebuild | scan counts -> list offsets | scan marks -> the
+//   scatter | every body into its place in cell order, cells ordered by body index (the list
+//   buffers' copy of the state, which the force kernels of the step read instead of the current
+//   one) | count neighbours closer than r_i + r_j + skin (keeping the first few), mark the spheres
+//   that can feel a force before the next rebuild | scan counts and marks -> list offsets, the
 //   marked spheres | write lists
 // Every barrier wait is bounded: a block that waits too long sets an error flag and returns.
 #pragma once
@@ -35,92 +35,146 @@ struct RebuildArgs {
     float *disp;
     int32_t *flags;
     unsigned int *bar;   // [0] arrivals, [1] generation
-    int32_t *blk;        // per-block partial sums (gridDim.x + 1)
+    unsigned long long *blk;   // per-block partial sums
     int32_t *err;
 };
 
-__device__ int block_sum(int v) {
-    __shared__ int ws[kRbBlock / 32];
+// Two 32-bit sums in one 64-bit word: both totals stay below 2^31, so no carry crosses.
+typedef unsigned long long Pair32;
+__device__ __forceinline__ Pair32 pair32(int lo, int hi) { return (Pair32)(uint32_t)lo | ((Pair32)(uint32_t)hi << 32); }
+
+// sum over the block, valid in every thread
+__device__ Pair32 block_sum(Pair32 v) {
+    __shared__ Pair32 ws[kRbBlock / 32];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
     __syncthreads();
-    int t = 0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < kRbBlock / 32; ++k) t += ws[k];
+    Pair32 t = 0;
+#pragma unroll
+    for (int k = 0; k < kRbBlock / 32; ++k) t += ws[k];
     __syncthreads();
-    return t;  // valid in thread 0
+    return t;
 }
 
-// inclusive scan across the block; *total receives the block total
-__device__ int block_incl_scan(int v, int *total) {
-    __shared__ int ws[kRbBlock / 32];
+// exclusive scan across the block; *total receives the block total
+__device__ Pair32 block_excl_scan(Pair32 v, Pair32 *total) {
+    __shared__ Pair32 ws[kRbBlock / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Pair32 x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
+        const Pair32 u = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += u;
     }
-    if (lane == 31) ws[w] = v;
+    if (lane == 31) ws[w] = x;
     __syncthreads();
-    if (w == 0) {
-        int x = (lane < kRbBlock / 32) ? ws[lane] : 0;
+    Pair32 before = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += u;
-        }
-        if (lane < kRbBlock / 32) ws[lane] = x;
+    for (int k = 0; k < kRbBlock / 32; ++k) {
+        if (k < w) before += ws[k];
+        all += ws[k];
     }
+    *total = all;
     __syncthreads();
-    const int r = v + (w > 0 ? ws[w - 1] : 0);
-    *total = ws[kRbBlock / 32 - 1];
-    __syncthreads();
-    return r;
+    return before + x - v;
 }
 
-// exclusive scan of in[0, m) into out[0, m], out[m] = total, by every block of a cooperative
-// grid of kRbBlock threads; blocks own contiguous chunks, blk holds gridDim.x + 1 partial sums.
-// The caller puts a grid barrier after it before reading out.
-__device__ bool grid_scan_raw(int32_t *blk, unsigned int *bar, int32_t *err, const int32_t *in,
-                              int32_t *out, int64_t m) {
-    const int64_t per = (m + gridDim.x - 1) / gridDim.x;
-    const int64_t b0 = (int64_t)blockIdx.x * per;
-    const int64_t b1 = (b0 + per < m) ? b0 + per : m;
-    int s = 0;
-    for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) s += in[i];
+// Exclusive scan of in[0, m) into out[0, m], out[m] = total, by every block of a cooperative
+// grid of kRbBlock threads (with in2: a second array of the same length beside it; in place is
+// allowed).  Blocks own contiguous chunks; blk holds a partial sum per block, which every block
+// adds up itself, so one grid barrier is enough.  The caller puts another after it before
+// reading out.  A thread takes kScanRun consecutive elements, two 16-byte loads.
+constexpr int kScanRun = 8;
+__device__ bool grid_scan_raw(Pair32 *blk, unsigned int *bar, int32_t *err, const int32_t *in,
+                              int32_t *out, int64_t m, const int32_t *in2 = nullptr,
+                              int32_t *out2 = nullptr) {
+    const int64_t per = ((m + gridDim.x - 1) / gridDim.x + kScanRun - 1) / kScanRun * kScanRun;
+    const int64_t b0 = min((int64_t)blockIdx.x * per, m);
+    const int64_t b1 = min(b0 + per, m);
+    Pair32 s = 0;
+    for (int64_t i = b0 + threadIdx.x; i < b1; i += kRbBlock) s += pair32(in[i], in2 ? in2[i] : 0);
     s = block_sum(s);
     if (threadIdx.x == 0) blk[blockIdx.x] = s;
     if (!grid_sync(bar, err)) return false;
-    if (blockIdx.x == 0) {
-        int run = 0;
-        for (int64_t base = 0; base < gridDim.x; base += blockDim.x) {
-            const int64_t i = base + threadIdx.x;
-            const int v = (i < gridDim.x) ? blk[i] : 0;
-            int tot;
-            const int incl = block_incl_scan(v, &tot);
-            if (i < gridDim.x) blk[i] = run + incl - v;
-            run += tot;
-        }
-        if (threadIdx.x == 0) out[m] = run;
+    Pair32 before = 0, all = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kRbBlock) {
+        const Pair32 v = __ldcg(blk + i);
+        all += v;
+        if (i < (int)blockIdx.x) before += v;
     }
-    if (!grid_sync(bar, err)) return false;
-    int run = blk[blockIdx.x];
-    for (int64_t base = b0; base < b1; base += blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        const int v = (i < b1) ? in[i] : 0;
-        int tot;
-        const int incl = block_incl_scan(v, &tot);
-        if (i < b1) out[i] = run + incl - v;
+    Pair32 run = block_sum(before);
+    if (blockIdx.x == 0) {
+        all = block_sum(all);
+        if (threadIdx.x == 0) {
+            out[m] = (int32_t)(uint32_t)all;
+            if (in2) out2[m] = (int32_t)(all >> 32);
+        }
+    }
+    auto load = [&](const int32_t *p, int64_t i, int v[kScanRun]) {
+        if (i + kScanRun <= b1) {
+#pragma unroll
+            for (int q = 0; q < kScanRun; q += 4) {
+                const int4 x = *reinterpret_cast<const int4 *>(p + i + q);
+                v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < kScanRun; ++q) v[q] = i + q < b1 ? p[i + q] : 0;
+        }
+    };
+    auto store = [&](int32_t *p, int64_t i, const int v[kScanRun]) {
+        if (i + kScanRun <= b1) {
+#pragma unroll
+            for (int q = 0; q < kScanRun; q += 4)
+                *reinterpret_cast<int4 *>(p + i + q) = make_int4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < kScanRun; ++q)
+                if (i + q < b1) p[i + q] = v[q];
+        }
+    };
+    for (int64_t base = b0; base < b1; base += kRbBlock * kScanRun) {
+        const int64_t i = base + (int64_t)threadIdx.x * kScanRun;
+        int v[kScanRun], v2[kScanRun];
+        load(in, i, v);
+        if (in2) load(in2, i, v2);
+        int a = 0, a2 = 0;
+#pragma unroll
+        for (int q = 0; q < kScanRun; ++q) {
+            a += v[q];
+            if (in2) a2 += v2[q];
+        }
+        Pair32 tot;
+        const Pair32 e = run + block_excl_scan(pair32(a, a2), &tot);
         run += tot;
+        int x = (int)(uint32_t)e, x2 = (int)(e >> 32);
+#pragma unroll
+        for (int q = 0; q < kScanRun; ++q) {
+            const int t = v[q];
+            v[q] = x;
+            x += t;
+            if (in2) {
+                const int t2 = v2[q];
+                v2[q] = x2;
+                x2 += t2;
+            }
+        }
+        store(out, i, v);
+        if (in2) store(out2, i, v2);
     }
     return true;
 }
 
-template <typename VT>
-__device__ __forceinline__ bool grid_scan(const RebuildArgs<VT> &a, const int32_t *in, int32_t *out,
-                                          int64_t m) {
-    return grid_scan_raw(a.blk, a.bar, a.err, in, out, m);
+// The place of body i in cell order, cells ordered by body index: its cell's offset and the number
+// of the cell's bodies with a smaller index (raw: every cell's bodies in the order their atomics
+// came).  Reads a handful of indexes, independent of one another.
+__device__ __forceinline__ int32_t ordered_slot(const int32_t *raw, const int32_t *cell_start,
+                                                int32_t key, int32_t i) {
+    const int b = cell_start[key], e = cell_start[key + 1];
+    int32_t slot = b;
+    for (int k = b; k < e; ++k) slot += raw[k] < i ? 1 : 0;
+    return slot;
 }
 
 // The cells within reach of body t (state in cell order): at most 3 x 3 rows of at most 3
@@ -263,28 +317,15 @@ __device__ bool rebuild_stages(const RebuildArgs<VT> &a) {
     }
     if (!grid_sync(a.bar, a.err)) return false;
     // 3. cell offsets
-    if (!grid_scan(a, a.cell_count, a.cell_start, a.ncell)) return false;
+    if (!grid_scan_raw(a.blk, a.bar, a.err, a.cell_count, a.cell_start, a.ncell)) return false;
     if (!grid_sync(a.bar, a.err)) return false;
     // 4. scatter
     for (int64_t i = g0; i < n; i += stride) a.sorted[a.cell_start[a.key[i]] + a.rank[i]] = (int32_t)i;
     if (!grid_sync(a.bar, a.err)) return false;
-    // 5. order each cell by body index (independent of the atomics' order)
-    for (int64_t c = g0; c < a.ncell; c += stride) {
-        const int b = a.cell_start[c], e = a.cell_start[c + 1];
-        for (int i = b + 1; i < e; ++i) {
-            const int32_t v = a.sorted[i];
-            int j = i - 1;
-            while (j >= b && a.sorted[j] > v) {
-                a.sorted[j + 1] = a.sorted[j];
-                --j;
-            }
-            a.sorted[j + 1] = v;
-        }
-    }
-    if (!grid_sync(a.bar, a.err)) return false;
-    // 6. gather into cell order
-    for (int64_t t = g0; t < n; t += stride) {
-        const int32_t b = a.sorted[t];
+    // 5. every body into its place, each cell ordered by body index (independent of the atomics'
+    // order)
+    for (int64_t b = g0; b < n; b += stride) {
+        const int64_t t = ordered_slot(a.sorted, a.cell_start, a.key[b], (int32_t)b);
         a.tmp.pr[t] = a.cur.pr[b];
         cp_vw((VT *)a.tmp.vw, t, (const VT *)a.cur.vw, b, n);
         a.tmp.tag[t] = a.cur.tag[b];
@@ -293,7 +334,7 @@ __device__ bool rebuild_stages(const RebuildArgs<VT> &a) {
         a.disp[t] = 0.f;
     }
     if (!grid_sync(a.bar, a.err)) return false;
-    // 7. neighbour counts; the first kListStash neighbours of each body are kept; the mark of
+    // 6. neighbour counts; the first kListStash neighbours of each body are kept; the mark of
     // every sphere that can feel a force before the next rebuild
     const double margin = 0.5 * a.skin * (1.0 + 1e-9);
     for (int64_t t = g0; t < n; t += stride) {
@@ -303,10 +344,8 @@ __device__ bool rebuild_stages(const RebuildArgs<VT> &a) {
         a.act[t] = list_marked(a.scenes[a.tmp.tag[t] >> 16], p, a.boxes, margin, k) ? 1 : 0;
     }
     if (!grid_sync(a.bar, a.err)) return false;
-    // 8. list offsets, and the marked spheres in ascending order
-    if (!grid_scan(a, a.cnt, a.start, n)) return false;
-    if (!grid_sync(a.bar, a.err)) return false;
-    if (!grid_scan(a, a.act, a.act, n)) return false;
+    // 7. list offsets, and the marked spheres in ascending order
+    if (!grid_scan_raw(a.blk, a.bar, a.err, a.cnt, a.start, n, a.act, a.act)) return false;
     if (!grid_sync(a.bar, a.err)) return false;
     for (int64_t t = g0; t < n; t += stride)
         if (a.act[t + 1] > a.act[t]) a.alist[a.act[t]] = (int32_t)t;
@@ -318,7 +357,7 @@ __device__ bool rebuild_stages(const RebuildArgs<VT> &a) {
         a.flags[4] = 1;
         a.flags[0] = 0;
     }
-    // 9. write the lists (if they fit; otherwise the force kernel searches the fresh grid):
+    // 8. write the lists (if they fit; otherwise the force kernel searches the fresh grid):
     // copied from the stash, or searched again for bodies with more neighbours than it holds
     if (need <= a.cap)
         for (int64_t t = g0; t < n; t += stride) {
