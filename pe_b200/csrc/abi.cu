@@ -219,6 +219,7 @@ int upload_tables(Ctx *c) {
         md[k].cdf = m.cdf;
         md[k].young = m.young;
         md[k].poisson = m.poisson;
+        md[k].round_f();
     }
     dfree(c, c->d_mats);
     c->d_mats = nullptr;

@@ -64,19 +64,16 @@ __device__ __forceinline__ T tmin(T a, T b) { return a < b ? a : b; }
 // response/DEMSolver.h:343-357); reff = r1 r2 / (r1 + r2) (contacttrait/DEMSolver.h:152-159)
 template <typename T>
 __device__ __forceinline__ void dem_contact(V3<T> n, T dist, V3<T> r1, V3<T> r2, V3<T> v1,
-                                            V3<T> w1, V3<T> v2, V3<T> w2, const MatDev &m1,
-                                            const MatDev &m2, bool self_is_1, Acc<T> &acc,
-                                            T reff = T(0)) {
+                                            V3<T> w1, V3<T> v2, V3<T> w2, const Coef<T> &q,
+                                            const MatDev &m1, const MatDev &m2, bool self_is_1,
+                                            Acc<T> &acc, T reff = T(0)) {
     // velFromWF, RigidBody.h:1080-1085
     const V3<T> rvel = (v1 + cross(w1, r1)) - (v2 + cross(w2, r2));
     // Contact.cpp:86-105: composed coefficients and the static/dynamic friction pick
-    const T k = T(1) / (T(m1.rk) + T(m2.rk));
-    const T cn = T(1) / (T(m1.rcn) + T(m2.rcn));
-    const T ct = T(1) / (T(m1.rct) + T(m2.rct));
+    const T k = q.k, cn = q.cn, ct = q.ct;
     const T nvel = dot(n, rvel);
     const T tvel = dot(n, rvel - n * nvel);
-    const T mu = (fabs(tvel) > T(kFrictionThreshold)) ? T(m1.cdf) + T(m2.cdf)
-                                                      : T(m1.csf) + T(m2.csf);
+    const T mu = (fabs(tvel) > T(kFrictionThreshold)) ? q.mu_d : q.mu_s;
     const T delta = -dist;
     const T relVelN = -nvel;
     const V3<T> relVel = -rvel;
@@ -152,6 +149,7 @@ struct DemArgs {
     // bank instead of through the body's tag)
     SceneInfo s0;
     MatDev m0;
+    Coef<VT> q0;      // and the coefficients of its contacts with itself
     // list step: the spheres marked at the last rebuild and their forces
     const int32_t *act = nullptr;     // exclusive offsets of the marks (n + 1)
     const int32_t *alist = nullptr;   // the marked spheres
@@ -192,11 +190,15 @@ __device__ __forceinline__ void pair_force_o(const DemArgs<VT> &a, const double4
     const double4 p1 = self1 ? pi : pj;
     const double4 p2 = self1 ? pj : pi;
     const double nx = p1.x - p2.x, ny = p1.y - p2.y, nz = p1.z - p2.z;
+    // apart by more than every rounding below: no square root
+    const double rs = p1.w + p2.w;
+    if (nx * nx + ny * ny + nz * nz > rs * rs * (1.0 + 1e-14)) return;
     const double len = length_rn(nx, ny, nz);
     const double dist = __dsub_rn(__dsub_rn(len, p1.w), p2.w);
     // only penetrating contacts produce a force (ContactBase.h:307-310)
     if (!(dist < -kContactThreshold)) return;
     const MatDev &mj = ONE ? a.m0 : a.mats[a.tag[j] & 0xffffu];
+    const Coef<T> q = ONE ? a.q0 : compose(mi, mj, T(0));
     const V3<T> vj = ld_vw(a.vw, a.n, j, 0), wj = ld_vw(a.vw, a.n, j, 1);
     V3<T> n, r1, r2;
     if (sizeof(T) == 8) {
@@ -219,9 +221,9 @@ __device__ __forceinline__ void pair_force_o(const DemArgs<VT> &a, const double4
     }
     const T reff = HERTZ ? (T(p1.w) * T(p2.w)) / (T(p1.w) + T(p2.w)) : T(0);
     if (self1)
-        dem_contact<T>(n, T(dist), r1, r2, vi, wi, vj, wj, mi, mj, true, acc, reff);
+        dem_contact<T>(n, T(dist), r1, r2, vi, wi, vj, wj, q, mi, mj, true, acc, reff);
     else
-        dem_contact<T>(n, T(dist), r1, r2, vj, wj, vi, wi, mj, mi, false, acc, reff);
+        dem_contact<T>(n, T(dist), r1, r2, vj, wj, vi, wi, q, mj, mi, false, acc, reff);
 }
 
 template <typename T, typename VT, bool HERTZ>
@@ -233,7 +235,7 @@ __device__ __forceinline__ void pair_force(const DemArgs<VT> &a, const double4 &
 
 // walls of the sphere's scene: planes (MaxContacts.h:777-790), then boxes
 // (MaxContacts.h:589-668); the sphere is body 1 and the fixed wall has zero velocity
-template <typename T, typename VT>
+template <typename T, typename VT, bool ONE = false>
 __device__ __forceinline__ void wall_forces(const DemArgs<VT> &a, const SceneInfo &s,
                                             const double4 &pi, V3<T> vi, V3<T> wi,
                                             const MatDev &mi, Acc<T> &acc) {
@@ -242,7 +244,13 @@ __device__ __forceinline__ void wall_forces(const DemArgs<VT> &a, const SceneInf
     const bool clear = pi.x - pi.w > s.wall_lo[0] && pi.x + pi.w < s.wall_hi[0] &&
                        pi.y - pi.w > s.wall_lo[1] && pi.y + pi.w < s.wall_hi[1] &&
                        pi.z - pi.w > s.wall_lo[2] && pi.z + pi.w < s.wall_hi[2];
-    const float pxf = float(pi.x), pyf = float(pi.y), pzf = float(pi.z), prf = float(pi.w);
+    float pxf = 0.f, pyf = 0.f, pzf = 0.f, prf = 0.f;
+    if (!clear) {
+        pxf = float(pi.x);
+        pyf = float(pi.y);
+        pzf = float(pi.z);
+        prf = float(pi.w);
+    }
     const float tol = 1e-3f * (1.0f + fabsf(pxf) + fabsf(pyf) + fabsf(pzf));
     for (int p = 0; p < (clear ? 0 : s.nplanes); ++p) {
         float4 pf;
@@ -260,7 +268,8 @@ __device__ __forceinline__ void wall_forces(const DemArgs<VT> &a, const SceneInf
         const double kk = dot_rn(pl.x, pl.y, pl.z, pi.x, pi.y, pi.z);
         const double dist = __dsub_rn(__dsub_rn(kk, pi.w), pl.w);
         if (!(dist < -kContactThreshold)) continue;
-        const MatDev &mw = a.mats[a.plane_mat[s.plane_begin + p]];
+        const MatDev &mw = ONE ? a.m0 : a.mats[a.plane_mat[s.plane_begin + p]];
+        const Coef<T> q = ONE ? a.q0 : compose(mi, mw, T(0));
         const V3<T> n = v3(T(pl.x), T(pl.y), T(pl.z));
         V3<T> r1;
         if (sizeof(T) == 8) {
@@ -270,7 +279,7 @@ __device__ __forceinline__ void wall_forces(const DemArgs<VT> &a, const SceneInf
         } else {
             r1 = n * (-(T(pi.w) + T(dist)));
         }
-        dem_contact<T>(n, T(dist), r1, zero, vi, wi, zero, zero, mi, mw, true, acc);
+        dem_contact<T>(n, T(dist), r1, zero, vi, wi, zero, zero, q, mi, mw, true, acc);
     }
     for (int k = 0; k < s.nboxes; ++k) {
         const double *B = a.boxes + 15 * (int64_t)(s.box_begin + k);
@@ -309,10 +318,11 @@ __device__ __forceinline__ void wall_forces(const DemArgs<VT> &a, const SceneInf
             gx = B[0] + qx; gy = B[1] + qy; gz = B[2] + qz;
         }
         if (!(dist < -kContactThreshold)) continue;
-        const MatDev &mw = a.mats[a.box_mat[s.box_begin + k]];
+        const MatDev &mw = ONE ? a.m0 : a.mats[a.box_mat[s.box_begin + k]];
+        const Coef<T> q = ONE ? a.q0 : compose(mi, mw, T(0));
         const V3<T> n = v3(T(nx), T(ny), T(nz));
         const V3<T> r1 = v3(T(gx - pi.x), T(gy - pi.y), T(gz - pi.z));
-        dem_contact<T>(n, T(dist), r1, zero, vi, wi, zero, zero, mi, mw, true, acc);
+        dem_contact<T>(n, T(dist), r1, zero, vi, wi, zero, zero, q, mi, mw, true, acc);
     }
 }
 
@@ -334,7 +344,7 @@ __device__ __forceinline__ double4 integrate_core(const DemArgs<VT> &a, int64_t 
     } else {
         // mixed precision: the same formulas in FP32 (SphereBase.h:169-171, 230-234)
         const float r = float(pi.w);
-        const float m = 4.0f / 3.0f * 3.14159265f * r * r * r * float(mi.density);
+        const float m = 4.0f / 3.0f * 3.14159265f * r * r * r * mi.density_f;
         im = T(__frcp_rn(m));
         ii = T(__frcp_rn(0.4f * m * r * r));
     }
@@ -805,7 +815,7 @@ __device__ __forceinline__ void contacts_loop(const DemArgs<VT> &a, bool rebuilt
                 pair_force_o<T, VT, HERTZ, ONE>(a, pi, vi, wi, mi, j0, a.pr[j0], (e0 >> 31) != 0u, acc);
             }
         }
-        wall_forces<T, VT>(a, s, pi, vi, wi, mi, acc);
+        wall_forces<T, VT, ONE>(a, s, pi, vi, wi, mi, acc);
         if constexpr (SPLIT) {
             // the integration of k_dem_move for this sphere
             uint32_t ext = ld_ext(a.vw, a.n, t);
@@ -1277,6 +1287,7 @@ void launch_list_shape(Ctx *c, const DemArgs<VT> &a, int contacts_done) {
         if (one) {
             b.s0 = c->scenes[0];
             b.m0 = c->mats_dev[0];
+            b.q0 = compose(b.m0, b.m0, VT(0));
             k_dem_contacts<VT, HERTZ, true, true, TRACKQ><<<gc, 128, 0, c->side>>>(b);
             k_dem_move<VT, TRACKQ, B, M, true, true><<<gm, B, 0, c->stream>>>(b);
         } else {
@@ -1318,6 +1329,7 @@ void launch_list_shape(Ctx *c, const DemArgs<VT> &a, int contacts_done) {
         DemArgs<VT> b = a;
         b.s0 = c->scenes[0];
         b.m0 = c->mats_dev[0];
+        b.q0 = compose(b.m0, b.m0, VT(0));
         if (!contacts_done) {
             cudaLaunchKernelEx(&cc, k_dem_contacts<VT, HERTZ, true>, b);
             c->launches++;
@@ -1359,6 +1371,7 @@ int launch_rebuild_contacts_t(Ctx *c, const DemArgs<VT> &a, int *fused) {
     if (ONE) {
         b.s0 = c->scenes[0];
         b.m0 = c->mats_dev[0];
+        b.q0 = compose(b.m0, b.m0, VT(0));
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);

@@ -50,7 +50,29 @@ struct MatDev {
     double rk, rcn, rct;   // 1/stiffness, 1/dampingN, 1/dampingT
     double csf, cdf;
     double young, poisson; // the extended Hertz law's effective modulus (Materials.h:586-600)
+    // the same in FP32, rounded once here instead of at every contact
+    float density_f, rk_f, rcn_f, rct_f, csf_f, cdf_f;
+    void round_f() {
+        density_f = (float)density;
+        rk_f = (float)rk; rcn_f = (float)rcn; rct_f = (float)rct;
+        csf_f = (float)csf; cdf_f = (float)cdf;
+    }
 };
+
+// The coefficients of a contact between two materials (Materials.h:633-715; static and dynamic
+// friction), in the arithmetic type of the step.
+template <typename T>
+struct Coef {
+    T k, cn, ct, mu_s, mu_d;
+};
+inline __host__ __device__ Coef<double> compose(const MatDev &a, const MatDev &b, double) {
+    return Coef<double>{1.0 / (a.rk + b.rk), 1.0 / (a.rcn + b.rcn), 1.0 / (a.rct + b.rct), a.csf + b.csf,
+                        a.cdf + b.cdf};
+}
+inline __host__ __device__ Coef<float> compose(const MatDev &a, const MatDev &b, float) {
+    return Coef<float>{1.0f / (a.rk_f + b.rk_f), 1.0f / (a.rcn_f + b.rcn_f), 1.0f / (a.rct_f + b.rct_f),
+                       a.csf_f + b.csf_f, a.cdf_f + b.cdf_f};
+}
 
 struct BodyBuf {
     double4 *pr = nullptr;

@@ -278,6 +278,7 @@ extern "C" int pe_b200_dem_step_static(int64_t n, const double *x, const double 
         md[k].rct = 1.0 / m.dampingT;
         md[k].csf = m.csf;
         md[k].cdf = m.cdf;
+        md[k].round_f();
     }
     double4 pl[kMaxPlanes];
     for (int p = 0; p < nplanes; ++p) {
