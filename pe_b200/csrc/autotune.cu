@@ -75,7 +75,8 @@ int set_tuning(Ctx *c, const Tuning &t, double skin) {
         return set_err(c, PE_B200_ERR_ARG, "invalid tuning");
     // captured list-step graphs bake the form in; the new form's first step runs outside a
     // capture (the split form creates its second stream there)
-    if (t.dem_split != c->tune.dem_split) {
+    if (c->form_auto || t.dem_split != c->tune.dem_split) {
+        c->form_auto = false;   // the caller's form from here on
         c->epoch++;
         c->nl.warm = false;
     }

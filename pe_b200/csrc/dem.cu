@@ -861,16 +861,9 @@ __global__ void __launch_bounds__(128) k_dem_contacts(DemArgs<VT> a0) {
 // SPLIT (the overlapped form): the kernel also integrates the marked spheres, and k_dem_move,
 // released at the trigger below, integrates the others meanwhile; it reads the rebuild flag
 // and the marks without waiting for this kernel, so they are made visible before the trigger.
-// resident blocks per SM the registers of the overlapped form's mixed-precision linear-law
-// kernels must allow: 4 (64 registers) took the contact-dense 1M step from 134 to 109 us (more
-// warps on the neighbours' loads); 5 and 6 spill too much (118, 147 us); the sparse step is the
-// same at all four.  The FP64 and Hertz kernels would spill kilobytes at 64 and keep their own.
-#ifndef PEB_FUSED_MINB
-#define PEB_FUSED_MINB 4
-#endif
-template <typename VT, bool HERTZ, bool ONE, bool SPLIT = false>
-__global__ void __launch_bounds__(kRbBlock,
-                                  (SPLIT && sizeof(VT) == 4 && !HERTZ) ? PEB_FUSED_MINB : 1)
+// MINB: resident blocks per SM the registers must allow (launch_rebuild_contacts).
+template <typename VT, bool HERTZ, bool ONE, bool SPLIT, int MINB>
+__global__ void __launch_bounds__(kRbBlock, MINB)
     k_rebuild_contacts(RebuildArgs<VT> ra, DemArgs<VT> da) {
     pdl_wait();
     const bool rebuilt = ra.flags[0] != 0;
@@ -1267,6 +1260,9 @@ bool split_streams(Ctx *c) {
     return true;
 }
 
+// the form of the list step (Tuning.dem_split), the caller's or the one picked for the scene
+int list_form(const Ctx *c) { return c->form_auto ? c->nl.form : c->tune.dem_split; }
+
 // contacts_done: the fused rebuild-and-contacts kernel has run (1: it stored the marked spheres'
 // forces; 2: the overlapped form, it integrates them too)
 template <typename VT, bool TRACKQ, int V, bool HERTZ>
@@ -1275,7 +1271,7 @@ void launch_list_shape(Ctx *c, const DemArgs<VT> &a, int contacts_done) {
     constexpr int B = kDemShapes[V].block;
     constexpr int M = sizeof(VT) == 4 ? kDemShapes[V].minb_f32 : kDemShapes[V].minb_f64;
     const bool one = c->nscenes == 1 && c->mats_dev.size() == 1 && !TRACKQ && !HERTZ;
-    if (c->tune.dem_split == 1 && !contacts_done && split_streams(c)) {
+    if (list_form(c) == 1 && !contacts_done && split_streams(c)) {
         // the marked spheres (forces and integration) on the second stream, beside the
         // integration of the others: both start once the rebuild kernel has finished, and the
         // next step waits for both
@@ -1350,12 +1346,12 @@ void launch_list_shape(Ctx *c, const DemArgs<VT> &a, int contacts_done) {
 // scheduled while the force kernel before it finishes.  *fused 0: not launched (the kernel
 // cannot be resident, or the driver refused it), the step runs the separate kernels; 1 or 2
 // (SPLIT, the overlapped form): launched.
-template <typename VT, bool HERTZ, bool ONE, bool SPLIT>
+template <typename VT, bool HERTZ, bool ONE, bool SPLIT, int MINB = 1>
 int launch_rebuild_contacts_t(Ctx *c, const DemArgs<VT> &a, int *fused) {
     ListBuf &L = c->nl;
     static int occ = 0;
     if (occ == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rebuild_contacts<VT, HERTZ, ONE, SPLIT>,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rebuild_contacts<VT, HERTZ, ONE, SPLIT, MINB>,
                                                           kRbBlock, 0) != cudaSuccess || occ < 1) {
             cudaGetLastError();
             occ = 0;
@@ -1384,7 +1380,7 @@ int launch_rebuild_contacts_t(Ctx *c, const DemArgs<VT> &a, int *fused) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = L.rebuild_pdl_off ? 1 : 2;
-    if (cudaLaunchKernelEx(&cfg, k_rebuild_contacts<VT, HERTZ, ONE, SPLIT>, ra, b) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, k_rebuild_contacts<VT, HERTZ, ONE, SPLIT, MINB>, ra, b) != cudaSuccess) {
         cudaGetLastError();
         L.fuse_off = true;
         return PE_B200_OK;
@@ -1402,8 +1398,19 @@ int launch_rebuild_contacts(Ctx *c, const DemArgs<VT> &a, bool ovl, int *fused) 
     const bool one = c->nscenes == 1 && c->mats_dev.size() == 1 && !track && !a.hertz;
     if (ovl && !track) {
         if (a.hertz) return launch_rebuild_contacts_t<VT, true, false, true>(c, a, fused);
-        return one ? launch_rebuild_contacts_t<VT, false, true, true>(c, a, fused)
-                   : launch_rebuild_contacts_t<VT, false, false, true>(c, a, fused);
+        // The overlapped form's linear-law kernels trade registers for warps, as the marked
+        // spheres' chains of dependent operations bound them: in FP64 two blocks of 256 threads
+        // per SM (405,224 spheres in contact: 62 us per step, 97 with one, 63 with three); in mixed
+        // precision three (97,336 spheres in contact: 15.3 us, 18.4 with four, 25.5 with five;
+        // 400,000 mostly apart: 10.3, 12.8, 17.4) until a fourth saves a whole pass over the
+        // spheres that outweighs its spills (1,048,576 in contact: 107 us with four, 115 with three).
+        constexpr int M = sizeof(VT) == 4 ? 3 : 2, MBIG = sizeof(VT) == 4 ? 4 : 2;
+        const bool big = c->n >= 600000;
+        if (one)
+            return big ? launch_rebuild_contacts_t<VT, false, true, true, MBIG>(c, a, fused)
+                       : launch_rebuild_contacts_t<VT, false, true, true, M>(c, a, fused);
+        return big ? launch_rebuild_contacts_t<VT, false, false, true, MBIG>(c, a, fused)
+                   : launch_rebuild_contacts_t<VT, false, false, true, M>(c, a, fused);
     }
     if (a.hertz) return launch_rebuild_contacts_t<VT, true, false, false>(c, a, fused);
     return one ? launch_rebuild_contacts_t<VT, false, true, false>(c, a, fused)
@@ -1427,9 +1434,9 @@ int list_step(Ctx *c, double dt) {
     // the rebuild check and the contact forces in one kernel (not while profiling, whose stage
     // timers keep the two apart, nor in the two-stream form)
     int fused = 0;
-    if (!L.coop_disabled && c->tune.rebuild_per_sm >= 0 && c->tune.dem_split != 1 && !c->prof &&
+    if (!L.coop_disabled && c->tune.rebuild_per_sm >= 0 && list_form(c) != 1 && !c->prof &&
         !L.fuse_off) {
-        rc = launch_rebuild_contacts<VT>(c, a, c->tune.dem_split == 2, &fused);
+        rc = launch_rebuild_contacts<VT>(c, a, list_form(c) == 2, &fused);
         if (rc) return rc;
     }
     if (fused) {
@@ -1604,6 +1611,7 @@ int list_capacity_check(Ctx *c) {
     ListBuf &L = c->nl;
     if (L.check_pending && cudaEventQuery(L.ev) == cudaSuccess) {
         L.check_pending = false;
+        L.entries = L.h_flags[2];
         if (L.h_flags[1]) {
             PEB_CUDA(c, cudaStreamSynchronize(c->stream));
             const int64_t need = std::max<int64_t>(L.h_flags[2], 0);
@@ -1696,6 +1704,29 @@ int capture_steps(Ctx *c, int32_t steps, double dt) {
 }
 
 }  // namespace
+
+// Picks the list step's form for a caller that did not: the overlapped one (2) or the plain one
+// (0); all give the same results.  Overlapping pays once the contact kernel, which then
+// integrates its spheres too, is long enough beside the integration of the others, and costs a
+// longer start (its release and the last block's wait).  One scene of one material, us per step
+// (plain / overlapped): FP64 mostly apart 100,000 spheres 6.6 / 6.3, 200,000 9.2 / 7.7, 700,000 21.7
+// / 19.1, 30,000 5.2 / 5.9; FP64 in contact (2 list entries a sphere or more) 2,197 11.5 / 10.9,
+// 97,336 23.8 / 22.5, 704,969 108 / 100; mixed mostly apart 400,000 10.5 / 10.3, 700,000 16.1 / 15.6,
+// 200,000 8.3 / 10.0; mixed in contact 29,791 11.9 / 10.8, 195,112 27.7 / 24.4, 1,048,576 134 / 107,
+// 8,000 10.3 / 10.5.  Batches of scenes stay plain (1.0M spheres in 64: 42.5 / 46.3).
+void dem_list_pick(Ctx *c) {
+    if (!c->form_auto) return;
+    const bool one = c->nscenes == 1 && c->mats.size() == 1 && !c->p.track_orientation &&
+                     c->p.force_model == 0;
+    const bool dense = c->nl.entries >= 2 * c->n;   // at the rebuild last read back
+    const bool fp64 = c->p.precision == PE_B200_FP64;
+    const bool over = dense ? fp64 || c->n >= 25000 : c->n >= (fp64 ? 100000 : 400000);
+    const int form = one && over ? 2 : 0;
+    if (form == c->nl.form) return;
+    c->nl.form = form;
+    c->epoch++;             // captured steps bake the form in
+    c->nl.warm = false;     // and its first step runs outside a capture
+}
 
 int dem_list_step(Ctx *c, double dt) {
     if (c->n == 0) return PE_B200_OK;

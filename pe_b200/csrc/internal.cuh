@@ -192,6 +192,8 @@ struct ListBuf {
     bool rebuild_pdl_off = false;  // the rebuild's cooperative launch without the early start
     bool warm = false;          // a list step has run since the buffers were (re)allocated
     int since_check = 1 << 20;  // steps since the last queued read-back of flags
+    int64_t entries = 0;        // list entries at the rebuild last read back
+    int form = 0;               // the step's form when the library picks it (dem_list_pick)
 };
 
 // launch shapes of the DEM list step, picked by pe_b200_autotune (autotune.cu)
@@ -307,6 +309,7 @@ struct Ctx {
     MBoxBuf mb;
     AdjState adj;
     Tuning tune;
+    bool form_auto = true;          // no tuning was set: the library picks the list step's form
     StepGraph sg;
     void *stage = nullptr;          // host-layout staging for uploads and downloads (transfer.cu)
     size_t stage_bytes = 0;
@@ -412,6 +415,7 @@ void dem_list_free(Ctx *c);
 int dem_list_request_rebuild(Ctx *c);
 int dem_list_rebuild_persistent(Ctx *c);
 int dem_list_step(Ctx *c, double dt);
+void dem_list_pick(Ctx *c);
 // runs whole graph replays of c->graph_steps list steps while they fit in nsteps; *done
 // receives the steps run (0 when graphs are off or not possible)
 int dem_list_graph_run(Ctx *c, int32_t nsteps, double dt, int32_t *done);
