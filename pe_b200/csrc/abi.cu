@@ -519,6 +519,7 @@ int pe_b200_destroy(pe_b200_ctx *h) {
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->ev_sort) cudaEventDestroy(c->ev_sort);
     if (c->dl) cudaStreamDestroy(c->dl);
     if (c->ev_dl0) cudaEventDestroy(c->ev_dl0);
     if (c->ev_dl1) cudaEventDestroy(c->ev_dl1);

@@ -437,6 +437,23 @@ __device__ __forceinline__ void box_cell(const double *gp, double x, double y, d
     cz = clampi((int)floor((z - gp[2]) * gp[3]), 0, (int)gp[6] - 1);
 }
 
+// inclusive prefix of cnt[0, n) in place, by the first warp of the block
+__device__ __forceinline__ void warp_prefix(int32_t *cnt, int n, int tid) {
+    if (tid >= 32) return;
+    int32_t run = 0;
+    for (int r0 = 0; r0 < n; r0 += 32) {
+        int32_t x = r0 + tid < n ? cnt[r0 + tid] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t u = __shfl_up_sync(0xffffffffu, x, o);
+            if (tid >= o) x += u;
+        }
+        x += run;
+        if (r0 + tid < n) cnt[r0 + tid] = x;
+        run = __shfl_sync(0xffffffffu, x, 31);
+    }
+}
+
 // Every contact of moving box m, visited by thread tid of the nthr threads of a block (all of
 // them call it): the spheres in the cells of the spheres' grid that the box's bounding box,
 // grown by the largest radius, covers; the scene's planes and fixed boxes; and (all_pairs:
@@ -466,8 +483,7 @@ __device__ void visit_box(const BoxArgs &a, int32_t m, int tid, int nthr, bool a
                 rcnt[r] = a.cell_start[c1] - rbeg[r];
             }
             __syncthreads();
-            if (tid == 0)
-                for (int r = 1; r < nr; ++r) rcnt[r] += rcnt[r - 1];   // inclusive prefix
+            warp_prefix(rcnt, nr, tid);
             __syncthreads();
             const int total = rcnt[nr - 1];
             for (int k = tid; k < total; k += nthr) {
@@ -514,8 +530,7 @@ __device__ void visit_box(const BoxArgs &a, int32_t m, int tid, int nthr, bool a
         nb_pre[tid] = cnt;
     }
     __syncthreads();
-    if (tid == 0)
-        for (int i = 1; i < 27; ++i) nb_pre[i] += nb_pre[i - 1];   // inclusive prefix
+    warp_prefix(nb_pre, 27, tid);
     __syncthreads();
     const int total = nb_pre[26];
     for (int g = tid; g < total; g += nthr) {
@@ -675,16 +690,21 @@ __global__ void k_sphere_box_forces(BoxArgs a, double *ext, const int32_t *list,
     }
 }
 
+// sums over the block in a fixed tree, valid in thread 0: halves of the block through shared memory
+// down to a warp, then within it
 __device__ void block_sum6(double *v, double (*sh)[6]) {
     const int t = threadIdx.x;
-    for (int k = 0; k < 6; ++k) sh[t][k] = v[k];
-    __syncthreads();
-    for (int half = kBoxBlk / 2; half > 0; half >>= 1) {
+    for (int half = kBoxBlk / 2; half >= 32; half >>= 1) {
+        if (t >= half && t < 2 * half)
+            for (int k = 0; k < 6; ++k) sh[t - half][k] = v[k];
+        __syncthreads();
         if (t < half)
-            for (int k = 0; k < 6; ++k) sh[t][k] += sh[t + half][k];
+            for (int k = 0; k < 6; ++k) v[k] += sh[t][k];
         __syncthreads();
     }
-    for (int k = 0; k < 6; ++k) v[k] = sh[0][k];
+    if (t < 32)
+        for (int o = 16; o > 0; o >>= 1)
+            for (int k = 0; k < 6; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
 }
 
 // Quaternion(phi, |phi|) * q (Quaternion.h:274-294, 1146-1153)
@@ -718,12 +738,15 @@ __device__ void box_advance(const BoxArgs &a, int32_t m, V v, V w, double dt, do
     wo[3 * m] = w.x; wo[3 * m + 1] = w.y; wo[3 * m + 2] = w.z;
 }
 
-// one block per moving box: its contact forces, then BoxTrait::move (boxtrait/Default.h:149-220)
-__global__ void __launch_bounds__(kBoxBlk) k_box_dem(BoxArgs a, double gx, double gy, double gz,
+// one block per moving box: its contact forces, then BoxTrait::move (boxtrait/Default.h:149-220).
+// Bound: the chain of its phases (a few thousand dependent cycles each), so residency counts for
+// more than registers: 40 steps of 110,592 spheres and 1,000 boxes with their transfers took 5.64
+// ms at 190 registers (two blocks per SM), 5.39 with three blocks, 5.05 with four, 4.86 with six.
+__global__ void __launch_bounds__(kBoxBlk, 6) k_box_dem(BoxArgs a, double gx, double gy, double gz,
                                                      double dt, double drag, int has_drag,
                                                      double *xo, double *qo, double *vo,
                                                      double *wo, int32_t *err) {
-    __shared__ double sh[kBoxBlk][6];
+    __shared__ double sh[kBoxBlk / 2][6];
     const int32_t m = blockIdx.x;
     const V xb = ld3(a.bx + 3 * m);
     const int32_t self = (int32_t)(a.n + m);
@@ -981,19 +1004,27 @@ __global__ void __launch_bounds__(kGridBlk) k_box_grid(int32_t m, const double *
         rext[wid] = ext;
     }
     __syncthreads();
-    if (t == 0) {
-        for (int w = 1; w < kGridBlk / 32; ++w) {
-            for (int a = 0; a < 3; ++a) {
-                rlo[a][0] = fmin(rlo[a][0], rlo[a][w]);
-                rhi[a][0] = fmax(rhi[a][0], rhi[a][w]);
-            }
-            rext[0] = fmax(rext[0], rext[w]);
+    if (wid == 0) {   // one lane per warp's values (32 of them)
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = rlo[a][lane];
+            hi[a] = rhi[a][lane];
         }
-        double h = fmax(2.0 * rext[0], rext[0] + rmax) + 4.0 * kContactThreshold;
+        ext = rext[lane];
+        for (int o = 16; o > 0; o >>= 1) {
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = fmin(lo[a], __shfl_down_sync(0xffffffffu, lo[a], o));
+                hi[a] = fmax(hi[a], __shfl_down_sync(0xffffffffu, hi[a], o));
+            }
+            ext = fmax(ext, __shfl_down_sync(0xffffffffu, ext, o));
+        }
+    }
+    static_assert(kGridBlk == 1024, "a value per lane");
+    if (t == 0) {
+        double h = fmax(2.0 * ext, ext + rmax) + 4.0 * kContactThreshold;
         if (!(h > 0.0 && h < 1e300)) h = 1.0;
         double span[3];
         for (int a = 0; a < 3; ++a) {
-            const double sp = rhi[a][0] - rlo[a][0];
+            const double sp = hi[a] - lo[a];
             span[a] = (sp >= 0.0 && sp < 1e300) ? sp : 0.0;   // non-finite states: one cell
         }
         int dim[3] = {1, 1, 1};
@@ -1011,7 +1042,7 @@ __global__ void __launch_bounds__(kGridBlk) k_box_grid(int32_t m, const double *
             dim[0] = dim[1] = dim[2] = 1;
             ncell = 1;
         }
-        for (int a = 0; a < 3; ++a) gp[a] = rlo[a][0];
+        for (int a = 0; a < 3; ++a) gp[a] = lo[a];
         gp[3] = 1.0 / h;
         for (int a = 0; a < 3; ++a) gp[4 + a] = dim[a];
         s_ncell = (int32_t)ncell;
@@ -1110,13 +1141,13 @@ BoxArgs box_args(Ctx *c) {
 }
 
 // this step's box rotations, bounding boxes and box grid
-int box_geometry(Ctx *c) {
+int box_geometry(Ctx *c, cudaStream_t st) {
     MBoxBuf &b = c->mb;
-    k_box_geom<<<grid_for(b.m, 128), 128, 0, c->stream>>>(b.m, b.x, b.q, b.len, b.R, b.aabb);
+    k_box_geom<<<grid_for(b.m, 128), 128, 0, st>>>(b.m, b.x, b.q, b.len, b.R, b.aabb);
     PEB_LAUNCHED(c);
     double rmax = 0.0;
     for (const SceneInfo &s : c->scenes) rmax = std::max(rmax, s.rmax);
-    k_box_grid<<<1, kGridBlk, 0, c->stream>>>(b.m, b.aabb, c->n > 0 ? rmax : 0.0, b.gparm, b.gcell,
+    k_box_grid<<<1, kGridBlk, 0, st>>>(b.m, b.aabb, c->n > 0 ? rmax : 0.0, b.gparm, b.gcell,
                                               b.gstart, b.gfill, b.gids, b.gnear);
     PEB_LAUNCHED(c);
     return PE_B200_OK;
@@ -1260,37 +1291,48 @@ void mbox_swap(Ctx *c) {
     std::swap(b.w, b.w2);
 }
 
-int mbox_dem(Ctx *c, double dt) {
+// The DEM step of the boxes, in three parts that dem_step places around its own kernels: the
+// geometry of the current state (it needs no sphere), the boxes' forces on the spheres (they need
+// both the geometry and the spheres' sort), and the boxes' own step (the same; it writes only the
+// boxes' next state).  `st`: the context's stream, or the side stream beside it.
+int mbox_dem_geometry(Ctx *c, cudaStream_t st) {
     MBoxBuf &b = c->mb;
-    if (b.m == 0) return PE_B200_OK;
-    const int64_t n = c->n;
-    const size_t nn = (size_t)std::max<int64_t>(n, 1);
-    if (b.ext_cap < n || !b.ext) {
+    const size_t nn = (size_t)std::max<int64_t>(c->n, 1);
+    if (b.ext_cap < c->n || !b.ext) {
         dfree(c, b.ext);
         b.ext = nullptr;
         PEB_CUDA(c, dmalloc(c, &b.ext, nn * 6 * sizeof(double) + (nn + 2) * sizeof(int32_t)));
-        b.ext_cap = n;
+        b.ext_cap = c->n;
     }
-    int32_t *near_list = (int32_t *)(b.ext + 6 * nn);
-    int32_t *near_count = near_list + nn;
-    int rc = box_geometry(c);
-    if (rc) return rc;
+    return box_geometry(c, st);
+}
+
+int mbox_dem_on_spheres(Ctx *c) {
+    MBoxBuf &b = c->mb;
+    const int64_t n = c->n;
+    if (n == 0) return PE_B200_OK;
+    int32_t *near_list = (int32_t *)(b.ext + 6 * (size_t)n);
+    int32_t *near_count = near_list + n;
     BoxArgs a = box_args(c);
     a.sorted = c->sorted;   // the grid step leaves the state in body order
-    if (n > 0) {
-        PEB_CUDA(c, cudaMemsetAsync(near_count, 0, sizeof(int32_t), c->stream));
-        k_sphere_box_near<<<grid_for(n, 256), 256, 0, c->stream>>>(a, b.ext, near_list, near_count);
-        PEB_LAUNCHED(c);
-        const int64_t warps = std::min<int64_t>(n, (int64_t)c->sm_count * 64);
-        k_sphere_box_forces<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(a, b.ext, near_list,
-                                                                              near_count);
-        PEB_LAUNCHED(c);
-    }
+    PEB_CUDA(c, cudaMemsetAsync(near_count, 0, sizeof(int32_t), c->stream));
+    k_sphere_box_near<<<grid_for(n, 256), 256, 0, c->stream>>>(a, b.ext, near_list, near_count);
+    PEB_LAUNCHED(c);
+    const int64_t warps = std::min<int64_t>(n, (int64_t)c->sm_count * 64);
+    k_sphere_box_forces<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(a, b.ext, near_list,
+                                                                          near_count);
+    PEB_LAUNCHED(c);
+    return PE_B200_OK;
+}
+
+int mbox_dem_boxes(Ctx *c, double dt, cudaStream_t st) {
+    MBoxBuf &b = c->mb;
+    BoxArgs a = box_args(c);
+    a.sorted = c->sorted;
     const int has_drag = c->p.damping < 1.0;
     const double drag = has_drag ? pow(c->p.damping, dt) : 1.0;
-    k_box_dem<<<b.m, kBoxBlk, 0, c->stream>>>(a, c->p.gravity[0], c->p.gravity[1],
-                                              c->p.gravity[2], dt, drag, has_drag, b.x2, b.q2,
-                                              b.v2, b.w2, c->d_err);
+    k_box_dem<<<b.m, kBoxBlk, 0, st>>>(a, c->p.gravity[0], c->p.gravity[1], c->p.gravity[2], dt, drag,
+                                       has_drag, b.x2, b.q2, b.v2, b.w2, c->d_err);
     PEB_LAUNCHED(c);
     return PE_B200_OK;
 }
@@ -1308,7 +1350,7 @@ int mbox_hc_count(Ctx *c, int32_t *total) {
     *total = 0;
     const MBoxBuf &b = c->mb;
     if (b.m == 0) return PE_B200_OK;
-    int rc = box_geometry(c);   // the state is in slot order here: sorted is the identity
+    int rc = box_geometry(c, c->stream);   // the state is in slot order here: sorted is the identity
     if (rc) return rc;
     k_box_count<<<b.m, kBoxBlk, 0, c->stream>>>(box_args(c), b.cnt);
     PEB_LAUNCHED(c);
@@ -1342,7 +1384,7 @@ int mbox_find_contacts(Ctx *c, std::vector<int64_t> &ids, std::vector<double> &g
     ids.clear();
     geom.clear();
     if (b.m == 0) return PE_B200_OK;
-    int rc = box_geometry(c);
+    int rc = box_geometry(c, c->stream);
     if (rc) return rc;
     BoxArgs a = box_args(c);
     a.sorted = c->sorted;   // the current state, binned by the grid just sorted

@@ -1040,8 +1040,9 @@ int launch_near(Ctx *c) {
     return PE_B200_OK;
 }
 
+// near_done: the candidate lists of this state are there
 template <typename VT>
-int launch_dem(Ctx *c, double dt) {
+int launch_dem(Ctx *c, double dt, bool near_done) {
     DemArgs<VT> a = dem_args<VT>(c, dt);
     prof_begin(c, ST_DEM);
     const unsigned g = grid_for(c->n, kDemBlock);
@@ -1057,8 +1058,10 @@ int launch_dem(Ctx *c, double dt) {
     } else {
         const float4 *pf = c->posf;
         const int32_t *nc = c->near, *ni = c->near + c->n;
-        const int rc = launch_near(c);
-        if (rc) return rc;
+        if (!near_done) {
+            const int rc = launch_near(c);
+            if (rc) return rc;
+        }
         if (a.hertz) {
             if (c->p.track_orientation) k_dem_near<VT, true, true><<<g, kDemBlock, 0, c->stream>>>(a, pf, nc, ni);
             else k_dem_near<VT, false, true><<<g, kDemBlock, 0, c->stream>>>(a, pf, nc, ni);
@@ -1244,7 +1247,8 @@ int list_rebuild(Ctx *c) {
     return PE_B200_OK;
 }
 
-// the second stream and the two events of the split list step, created on first use
+// the second stream and the events of the split list step and of the moving boxes, created on
+// first use
 bool split_streams(Ctx *c) {
     if (c->side) return true;
     if (c->split_failed) return false;
@@ -1252,7 +1256,8 @@ bool split_streams(Ctx *c) {
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
     if (cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, hi) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_sort, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
         c->split_failed = true;
         return false;
@@ -1505,21 +1510,58 @@ int dem_search(Ctx *c) {
     return rc ? rc : launch_near(c);
 }
 
+namespace {
+// One grid step of a scene with moving boxes.  The boxes' geometry and grid (one block) and their
+// own step run on the side stream beside the spheres' sort, candidate lists and forces, which they
+// do not depend on: 110,592 spheres with 1,000 boxes took 160 us a step one after the other.  The
+// context's stream waits for the side stream before the step ends, so nothing else ever runs
+// beside it; without a side stream everything runs on the context's.
+int dem_step_boxes(Ctx *c, double dt) {
+    const bool fork = split_streams(c);
+    cudaStream_t side = fork ? c->side : c->stream;
+    auto order = [&](cudaEvent_t ev, cudaStream_t first, cudaStream_t then) -> int {
+        if (!fork) return PE_B200_OK;
+        PEB_CUDA(c, cudaEventRecord(ev, first));
+        PEB_CUDA(c, cudaStreamWaitEvent(then, ev, 0));
+        return PE_B200_OK;
+    };
+    auto body = [&]() -> int {
+        int rc = order(c->ev_fork, c->stream, side);
+        if (!rc) rc = mbox_dem_geometry(c, side);
+        if (rc) return rc;
+        const bool lists = c->tune.dem_grid != 1;
+        if (c->n > 0) {
+            rc = dem_sort(c, lists);
+            if (rc) return rc;
+        }
+        rc = order(c->ev_join, side, c->stream);           // geometry -> forces on the spheres
+        if (!rc) rc = order(c->ev_sort, c->stream, side);  // sort -> the boxes' step
+        if (!rc) rc = mbox_dem_boxes(c, dt, side);
+        if (!rc && c->n > 0 && lists) rc = launch_near(c);
+        if (!rc) rc = mbox_dem_on_spheres(c);
+        if (!rc && c->n > 0) rc = launch_dem<double>(c, dt, lists);   // boxes: FP64 only
+        return rc ? rc : order(c->ev_join, side, c->stream);
+    };
+    const int rc = body();
+    if (rc) {
+        if (fork) cudaStreamSynchronize(c->side);   // nothing of a failed step stays behind
+        return rc;
+    }
+    if (c->n > 0) std::swap(c->cur, c->nxt);
+    mbox_swap(c);
+    return PE_B200_OK;
+}
+}  // namespace
+
 int dem_step(Ctx *c, double dt) {
-    int rc;
-    if (c->n > 0) {
-        rc = dem_sort(c, c->tune.dem_grid != 1);
-        if (rc) return rc;
-    }
-    // moving boxes: their forces on the spheres and their own step, from the current state
-    rc = mbox_dem(c, dt);
+    if (c->mb.m > 0) return dem_step_boxes(c, dt);
+    if (c->n == 0) return PE_B200_OK;
+    int rc = dem_sort(c, c->tune.dem_grid != 1);
     if (rc) return rc;
-    if (c->n > 0) {
-        rc = (c->p.precision == PE_B200_FP64) ? launch_dem<double>(c, dt) : launch_dem<float>(c, dt);
-        if (rc) return rc;
-        std::swap(c->cur, c->nxt);
-    }
-    if (c->mb.m > 0) mbox_swap(c);
+    rc = (c->p.precision == PE_B200_FP64) ? launch_dem<double>(c, dt, false)
+                                          : launch_dem<float>(c, dt, false);
+    if (rc) return rc;
+    std::swap(c->cur, c->nxt);
     return PE_B200_OK;
 }
 

@@ -248,6 +248,7 @@ struct Ctx {
     // and its fork and join events
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_sort = nullptr;  // moving boxes: the spheres' sort, for the side stream
     bool split_failed = false;
     // a second stream for the copies of a download (transfer.cu), created on first use
     cudaStream_t dl = nullptr;
@@ -453,7 +454,9 @@ int mbox_download(Ctx *c, double *x, double *q, double *v, double *w);
 void mbox_free(Ctx *c);
 // DEM: the boxes' forces on the spheres (mb.ext, by body index of the current buffers) and
 // the boxes' own step into the next box buffers; the caller swaps them after the sphere step
-int mbox_dem(Ctx *c, double dt);
+int mbox_dem_geometry(Ctx *c, cudaStream_t st);
+int mbox_dem_on_spheres(Ctx *c);
+int mbox_dem_boxes(Ctx *c, double dt, cudaStream_t st);
 void mbox_swap(Ctx *c);
 // HCSITS (bodies n .. n+m-1 after the spheres): body cache, contacts (count, then write after
 // the sphere contacts), integration
