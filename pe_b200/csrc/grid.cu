@@ -9,10 +9,9 @@
 //   scatter(slot of body i = cell_start[key[i]] + rank[i])
 //   order  (each cell by body index, so the result is independent of atomic order; a body finds
 //           its place from the indexes of its cell's bodies)
-// Outside graph captures they run in one cooperative kernel (k_grid_sort) with bounded grid
-// barriers between them, which also clears the counts for the next step; in a capture, and with
-// rebuild_per_sm = -1 (no cooperative launches), they run as separate kernels.  Both give the
-// same arrays.
+// They run in one cooperative kernel (k_grid_sort) with bounded grid barriers between them, which
+// also clears the counts for the next step; with rebuild_per_sm = -1 (no cooperative launches), as
+// separate kernels.  Both give the same arrays.
 #include "rebuild.cuh"
 
 namespace peb {
@@ -129,6 +128,14 @@ __global__ void k_order(int64_t n, const int32_t *__restrict__ raw, const int32_
     if (i < n) order_body((int32_t)i, raw, start, key, sorted, pr, tag, scenes, posf);
 }
 
+// the whole of scan_exclusive in one cooperative grid
+__global__ void __launch_bounds__(kRbBlock) k_scan_grid(const int32_t *in, int32_t *out, int64_t n,
+                                                        unsigned long long *blk, unsigned int *bar,
+                                                        int32_t *err, const int32_t *cond) {
+    if (cond && !*cond) return;
+    grid_scan_raw(blk, bar, err, in, out, n);
+}
+
 struct GridSortArgs {
     int64_t n, ncell;
     int32_t *cell_count, *cell_start, *key, *rank, *raw, *sorted;
@@ -179,8 +186,27 @@ int scan_exclusive(Ctx *c, const int32_t *in, int32_t *out, int64_t n) {
     return scan_exclusive_cond(c, in, out, n, nullptr);
 }
 
-// cond (device int, may be null): when it holds 0 every kernel of the scan returns at once
+// cond (device int, may be null): when it holds 0 every kernel of the scan returns at once.  One
+// cooperative kernel with one grid barrier (a chunk of a few runs per thread; the kernels that
+// follow it see the end of the launch as the second), or, where those are refused or turned off,
+// tiles, tile sums and their addition as separate kernels: in, out and the totals are the same.
 int scan_exclusive_cond(Ctx *c, const int32_t *in, int32_t *out, int64_t n, const int32_t *cond) {
+    if (n > 0 && c->gs_blk && !c->gs_coop_off && c->tune.rebuild_per_sm >= 0) {
+        const unsigned grid = (unsigned)std::min<int64_t>(
+            std::min<int64_t>((n + kRbBlock * kScanRun - 1) / (kRbBlock * kScanRun), c->sm_count),
+            c->gs_blk_cap - 1);
+        unsigned long long *blk = c->gs_blk;
+        unsigned int *bar = c->gs_bar;
+        int32_t *err = c->d_err;
+        void *args[] = {&in, &out, &n, &blk, &bar, &err, &cond};
+        if (cudaLaunchCooperativeKernel((const void *)k_scan_grid, dim3(grid), dim3(kRbBlock), args, 0,
+                                        c->stream) == cudaSuccess) {
+            c->launches++;
+            return PE_B200_OK;
+        }
+        cudaGetLastError();
+        c->gs_coop_off = true;
+    }
     // recursive reduce-then-scan; scratch holds every level's tile sums
     std::vector<int64_t> sizes;
     int64_t m = n;
@@ -279,15 +305,7 @@ int grid_bin_current(Ctx *c) {
 // cell_count is cleared for the producing kernel of this step.
 int grid_sort(Ctx *c, bool with_pos) {
     prof_begin(c, ST_SORT);
-    // one cooperative kernel for steps launched one by one; inside a graph capture the separate
-    // kernels (cheap to launch from a graph) measured faster than the kernel's grid barriers
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess) {
-        cudaGetLastError();
-        cap = cudaStreamCaptureStatusActive;
-    }
-    if (cap == cudaStreamCaptureStatusNone && !c->gs_coop_off && c->gs_blk &&
-        c->tune.rebuild_per_sm >= 0 && c->ncell > 0) {
+    if (!c->gs_coop_off && c->gs_blk && c->tune.rebuild_per_sm >= 0 && c->ncell > 0) {
         static int occ = 0;
         if (occ == 0 &&
             (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_grid_sort, kRbBlock, 0) !=
