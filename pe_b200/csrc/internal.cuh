@@ -170,7 +170,7 @@ struct ListBuf {
     int32_t *idx = nullptr;     // cap
     float *disp = nullptr;      // path length since the last rebuild
     int32_t *flags = nullptr;   // [0] rebuild requested, [1] list overflowed at this rebuild,
-                                // [2] entries needed, [3] rebuild count
+                                // [2] entries needed, [3] rebuild count, [4] this step rebuilt
     int32_t *h_flags = nullptr; // pinned mirror
     cudaEvent_t ev = nullptr;
     bool check_pending = false;
@@ -188,6 +188,8 @@ struct ListBuf {
     unsigned long long *rb_blk = nullptr;
     int64_t rb_blk_cap = 0;
     bool coop_disabled = false;
+    unsigned int *steps_bar = nullptr;   // the steps kernel's barrier words (dem.cu)
+    bool steps_off = false;  // it cannot be launched here
     bool fuse_off = false;   // the fused rebuild-and-contacts kernel cannot be launched here
     bool rebuild_pdl_off = false;  // the rebuild's cooperative launch without the early start
     bool warm = false;          // a list step has run since the buffers were (re)allocated
