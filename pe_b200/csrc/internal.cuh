@@ -108,6 +108,7 @@ struct NbgsBuf {
     bool staged_off = false;                  // nor the grid form with staged contacts
     bool on_device = false;                   // the last step's counts are only on the device
     bool plan_none = false;                   // queued steps planned without contacts
+    bool plan_few = false;                    // or for a few (what one thread colours)
     bool warm = false;                        // a queued step has run on these buffers
     // captured CUDA graphs of queued steps, each valid for the buffers, settings, plan and
     // sweep grid in its key (nbgs.cu nbgs_graph_run); a miss replaces the least recently used

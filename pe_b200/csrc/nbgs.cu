@@ -2613,14 +2613,15 @@ inline int64_t queued_sweep_blocks(const Ctx *c) {
 template <typename VT>
 int launch_sweeps_queued(Ctx *c, int model, bool gen, int iters, int64_t cap, VT dtinv,
                          const Cache<VT> &cc, const BodyV<VT> &bv, int64_t n,
-                         unsigned long long *dl) {
+                         unsigned long long *dl, bool few) {
     NbgsBuf &nb = c->nb;
     int32_t *dd = nb.dd;
     const int mode = c->tune.nbgs_sweeps;
     if (mode == 0 && !gen) {
         // a few contacts: the compact form; more: the form without barriers
-        bool done = false;
-        int rc = launch_sweeps_flow<VT>(c, model, gen, iters, 7, cap, dtinv, cc, bv, 0, dl, &done);
+        bool done = few;
+        int rc = few ? PE_B200_OK
+                     : launch_sweeps_flow<VT>(c, model, gen, iters, 7, cap, dtinv, cc, bv, 0, dl, &done);
         if (rc) return rc;
         if (done) {
             rc = launch_sweeps_compact<VT>(c, model, iters, 8, dtinv, cc, bv, 0, dl, &done);
@@ -2732,6 +2733,9 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     int rc = nbgs_alloc(c, auto_cap);
     if (rc) return rc;
     nb.on_device = queued;
+    // planned for a few contacts: the stages only more of them need are left out (the colouring's
+    // adjacency and rounds, the sweeps without barriers)
+    const bool few = queued && nb.plan_few && c->tune.nbgs_sweeps == 0;
     // 1. sort, permute to slot order, body cache
     if (n > 0) {
         if (!c->binned) {
@@ -2789,7 +2793,9 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         } else {
             PEB_CUDA(c, cudaMemsetAsync(nb.cnt, 0, sizeof(int32_t), c->stream));
         }
-        const PlanArgs pa{nb.cnt + n, nb.cap, colour_serial_max(c), dd, nb.color, nb.body_cnt, nb.rem,
+        // a step planned for a few contacts aborts beyond what one thread colours
+        const int64_t limit = few ? std::min<int64_t>(nb.cap, colour_serial_max(c)) : nb.cap;
+        const PlanArgs pa{nb.cnt + n, limit, colour_serial_max(c), dd, nb.color, nb.body_cnt, nb.rem,
                           nb.flags, nb.used, nbod, nbod, 2 * kMaxColors};
         k_plan<<<capped_grid(c, std::max<int64_t>(nbod, kMaxRounds), kBlk), kBlk, 0, c->stream>>>(pa);
         PEB_LAUNCHED(c);
@@ -2848,7 +2854,7 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     const bool any = queued ? !nb.plan_none : nc > 0;
     // the sweeps without barriers may run: k_cache writes the bodies' contacts in colour order
     // (over the colouring's adjacency, which it no longer needs)
-    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && (queued || gen || nc > kCompactMax)
+    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && !few && (queued || gen || nc > kCompactMax)
                             ? nb.body_adj : nullptr;
     if (any) {
         prof_begin(c, ST_COLOR);
@@ -2858,7 +2864,7 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         // the body -> contacts adjacency of the parallel rounds (skipped on the device, or by the
         // host, when one thread colours the step)
         const int32_t *rounds = queued ? dd + kDdRounds : nullptr;
-        if (queued || nc > serial_max || flow_adj) {
+        if ((queued && !few) || nc > serial_max || flow_adj) {
             if (!queued)   // k_plan cleared it, and the arrays below
                 PEB_CUDA(c, cudaMemsetAsync(nb.body_cnt, 0, ((size_t)nbod + 1) * sizeof(int32_t), c->stream));
             k_degree<<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, rounds, raw.b1, raw.b2, nb.body_cnt);
@@ -2885,8 +2891,10 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
                 ncp, dd, serial_max, raw.b1, raw.b2, nb.color, nbod, nb.used, in_smem ? 1 : 0,
                 c->d_err);
             PEB_LAUNCHED(c);
-            rc = launch_color_rounds(c, ncp, dd, raw, cap, serial_max);
-            if (rc) return rc;
+            if (!few) {
+                rc = launch_color_rounds(c, ncp, dd, raw, cap, serial_max);
+                if (rc) return rc;
+            }
         } else {
             int round = 0;
             if (nc <= serial_max) {
@@ -2955,7 +2963,7 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     if (c->want_residual) PEB_CUDA(c, cudaMemsetAsync(nb.red, 0, 2 * sizeof(double), c->stream));
     if (queued && any && iters > 0) {
         prof_begin(c, ST_SWEEP);
-        rc = launch_sweeps_queued<VT>(c, model, gen, iters, cap, VT(1.0 / dt), cc, bv, n, dl);
+        rc = launch_sweeps_queued<VT>(c, model, gen, iters, cap, VT(1.0 / dt), cc, bv, n, dl, few);
         if (rc) return rc;
         prof_end(c, ST_SWEEP);
     } else if (!queued && nc > 0) {
@@ -3189,7 +3197,7 @@ int nbgs_graph_run(Ctx *c, int32_t nsteps, double dt, int32_t *ran) {
     const uint64_t key[12] = {(uint64_t)(uintptr_t)c->cur.pr, (uint64_t)(uintptr_t)c->nxt.pr,
                               (uint64_t)(uintptr_t)nb.cache, (uint64_t)nb.cap, c->epoch,
                               (uint64_t)c->p.max_iterations, (uint64_t)c->p.relaxation_model,
-                              erpu.u, dtu.u, (uint64_t)nb.plan_none,
+                              erpu.u, dtu.u, (uint64_t)nb.plan_none | (uint64_t)nb.plan_few << 1,
                               (uint64_t)queued_sweep_blocks(c), (uint64_t)gs};
     NbgsBuf::GraphSlot *hit = nullptr, *lru = &nb.gslot[0];
     for (NbgsBuf::GraphSlot &s : nb.gslot) {
@@ -3279,6 +3287,8 @@ int nbgs_run(Ctx *c, int32_t nsteps, double dt) {
             // the next call's steps skip the contact stages while the scene has no contacts:
             // none in any step of this call
             nb.plan_none = nb.h_dd[kDdSeen] == 0;
+            // and are planned for a few while every step of the call had few
+            nb.plan_few = !nb.plan_none && nb.h_dd[kDdSeen] <= colour_serial_max(c) * 3 / 4;
             break;
         }
         const int32_t done = nb.h_dd[kDdSteps];
@@ -3290,7 +3300,7 @@ int nbgs_run(Ctx *c, int32_t nsteps, double dt) {
             int rc = nbgs_alloc(c, need + need / 4 + 1024);
             if (rc) return rc;
         }
-        nb.plan_none = false;
+        nb.plan_none = nb.plan_few = false;
         PEB_CUDA(c, cudaMemsetAsync(nb.dd + kDdAbort, 0, sizeof(int32_t), c->stream));
         nb.h_dd[kDdAbort] = 0;
         left -= done;
