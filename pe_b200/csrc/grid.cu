@@ -12,6 +12,7 @@
 // They run in one cooperative kernel (k_grid_sort) with bounded grid barriers between them, which
 // also clears the counts for the next step; with rebuild_per_sm = -1 (no cooperative launches), as
 // separate kernels.  Both give the same arrays.
+#include "near.cuh"
 #include "rebuild.cuh"
 
 namespace peb {
@@ -105,7 +106,8 @@ __global__ void k_scatter(int64_t n, const int32_t *__restrict__ key,
 }
 
 // body i into its place in cell order, and (posf) its FP32 record: the position relative to its
-// scene's grid origin and the radius (the candidate records of the grid DEM step)
+// scene's grid origin and the radius with the margin of near_margin added (the candidate records of
+// the grid DEM step)
 __device__ __forceinline__ void order_body(int32_t i, const int32_t *__restrict__ raw,
                                            const int32_t *__restrict__ start,
                                            const int32_t *__restrict__ key, int32_t *sorted,
@@ -117,7 +119,8 @@ __device__ __forceinline__ void order_body(int32_t i, const int32_t *__restrict_
     if (!posf) return;
     const double4 p = pr[i];
     const SceneInfo &s = scenes[tag[i] >> 16];
-    posf[t] = make_float4(float(p.x - s.lo[0]), float(p.y - s.lo[1]), float(p.z - s.lo[2]), float(p.w));
+    const float x = float(p.x - s.lo[0]), y = float(p.y - s.lo[1]), z = float(p.z - s.lo[2]), r = float(p.w);
+    posf[t] = make_float4(x, y, z, r + near_margin(x, y, z, r));
 }
 
 __global__ void k_order(int64_t n, const int32_t *__restrict__ raw, const int32_t *__restrict__ start,

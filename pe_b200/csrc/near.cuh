@@ -11,6 +11,12 @@ namespace peb {
 
 constexpr int kNear = 16;   // recorded candidates per sphere; one with more searches its cells
 
+// What a sphere's rounded FP32 record may be off: |d_fp32 - d| stays below ~1e-7 (|x| + |y| + |z| + 2 r +
+// d) for any partner closer than r_i + r_j; the margin is 100 times that.
+__device__ __forceinline__ float near_margin(float x, float y, float z, float r) {
+    return 1e-5f * (1.0f + fabsf(x) + fabsf(y) + fabsf(z) + 4.0f * r);
+}
+
 // slot t's recorded candidates in ascending order, the order in which a 27-cell scan visits them
 // (a sorting network over registers; the places from cnt on hold INT_MAX and sort last)
 __device__ __forceinline__ void load_near(const int32_t *__restrict__ near_idx, int64_t n, int64_t t,
