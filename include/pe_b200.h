@@ -248,13 +248,14 @@ typedef struct {
     double skin;             /* neighbour-list skin (cells are re-planned to 2 r_max + skin) */
     double ms_per_step;      /* pe_b200_autotune: measured time of the winner; else -1 */
     int32_t variants;        /* output: number of launch shapes */
-    int32_t nbgs_sweeps;     /* HCSITS sweeps: 0 automatic (4 when every colour fits one
-                                block, else 5 when the bodies fit, else 2), 1 one thread-block
-                                cluster with hardware barriers, 2 one cooperative grid with
-                                barriers through global memory, 3 one launch per colour, 4 one
-                                thread block with __syncthreads between colours (when every
-                                colour fits it), 5 one cluster with the bodies' records in its
-                                distributed shared memory (sphere scenes whose bodies fit) */
+    int32_t nbgs_sweeps;     /* HCSITS sweeps: 0 automatic (a block for up to 768 contacts of a
+                                sphere scene, else each contact waits for its two bodies only, all
+                                in one cooperative grid), 1 one thread-block cluster with hardware
+                                barriers, 2 one cooperative grid with barriers through global
+                                memory, 3 one launch per colour, 4 one thread block with
+                                __syncthreads between colours (when every colour fits it), 5 one
+                                cluster with the bodies' records in its distributed shared memory
+                                (sphere scenes whose bodies fit); all give the same results */
     int32_t dem_grid;        /* DEM grid step (cell search every step): 0 candidates read from an
                                 FP32 position copy in cell order, with an exact FP64 test for the
                                 close ones; 1 every candidate through its FP64 record (the same
@@ -265,7 +266,9 @@ typedef struct {
                                 overlap on one stream: the kernel that checks for (and runs) the
                                 rebuild lets the integration of the unmarked spheres start, then
                                 computes and integrates the marked ones (orientation tracking
-                                runs form 0).  All forms give the same results */
+                                runs form 0).  All forms give the same results.  While no tuning
+                                was set the library picks between 0 and 2 by size, precision and
+                                list density, and runs the steps of small scenes in one kernel */
 } pe_b200_tuning;
 int pe_b200_get_tuning(pe_b200_ctx *ctx, pe_b200_tuning *out);
 int pe_b200_set_tuning(pe_b200_ctx *ctx, const pe_b200_tuning *t);

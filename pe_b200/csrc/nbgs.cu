@@ -1732,7 +1732,7 @@ __global__ void __launch_bounds__(kDsBlk) k_sweeps_dsmem(int iters, const int32_
 // itself (700 cycles in FP64 without friction, 1100 in FP32 with it), its store into the L2 and the
 // poll that sees it (a lone store and poll take 470 cycles within a die and 850 across, a poll of
 // a warp's mailboxes about 900).  100 sweeps of 8 colours: 1.26 ms in FP32 with friction (50,000
-// contacts, 2.2 ms with staged records and a grid barrier) and 1.28 ms in FP64 without (32,000
+// contacts, 2.2 ms with staged records and a grid barrier) and 1.12 ms in FP64 without (32,000
 // contacts, 3.0 ms in one cluster's shared memory); 39 colours of a box stack: 5.5 ms against 7.3
 // in one block.  Polling through one small tag per mailbox before loading it was slower (1.63 and
 // 1.49 ms): the traffic of the polls is not what bounds it.
