@@ -2854,7 +2854,12 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     const bool any = queued ? !nb.plan_none : nc > 0;
     // the sweeps without barriers may run: k_cache writes the bodies' contacts in colour order
     // (over the colouring's adjacency, which it no longer needs)
-    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && !few && (queued || gen || nc > kCompactMax)
+    // Host-driven steps with fewer contacts stay in one block, whose hops through shared memory are
+    // shorter while it has few contacts to run: stacks of boxes, us per step (this / one block)
+    // without friction 2x2x2 1594 / 1199, 5x5x5 4245 / 4055, 6x6x6 5133 / 5745; with friction 3x3x3
+    // (93 contacts at the end) 3260 / 3152, 2x4x4 (145) 3373 / 3501, 6x6x6 6242 / 7910.
+    const int64_t flow_min = gen && c->p.relaxation_model != PE_B200_INELASTIC_FRICTIONLESS ? 96 : kCompactMax;
+    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && !few && (queued || nc > flow_min)
                             ? nb.body_adj : nullptr;
     if (any) {
         prof_begin(c, ST_COLOR);
