@@ -2858,7 +2858,8 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     // shorter while it has few contacts to run: stacks of boxes, us per step (this / one block)
     // without friction 2x2x2 1594 / 1199, 5x5x5 4245 / 4055, 6x6x6 5133 / 5745; with friction 3x3x3
     // (93 contacts at the end) 3260 / 3152, 2x4x4 (145) 3373 / 3501, 6x6x6 6242 / 7910.
-    const int64_t flow_min = gen && c->p.relaxation_model != PE_B200_INELASTIC_FRICTIONLESS ? 96 : kCompactMax;
+    const int64_t flow_min = !gen ? kCompactMax
+                             : c->p.relaxation_model == PE_B200_INELASTIC_FRICTIONLESS ? 1100 : 96;
     int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && !few && (queued || nc > flow_min)
                             ? nb.body_adj : nullptr;
     if (any) {
