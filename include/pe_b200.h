@@ -325,7 +325,8 @@ int pe_b200_validate(pe_b200_ctx *ctx, int64_t *problems);
 /* Self-test of the bounded device waits: launches one kernel that waits on a flag nothing sets,
  * which gives up after `polls` polls (1 <= polls <= 2^24) and records a timeout.  Returns
  * PE_B200_ERR_TIMEOUT, as a real barrier or peer wait that ran out would, and leaves the context
- * usable. */
+ * usable; what such a wait leaves behind in the context's grid barriers is left there first, and
+ * another code is returned if reporting the timeout did not clear it. */
 int pe_b200_selftest_timeout(pe_b200_ctx *ctx, int64_t polls);
 
 /* Number of kernels this context launched since creation (device-side work accounting). */

@@ -881,6 +881,10 @@ static int check_device_errors(Ctx *c) {
     const int32_t e = *c->h_err;
     if (e) {
         PEB_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int32_t), c->stream));
+        if (e & DERR_TIMEOUT) {
+            const int rc = reset_barriers(c);
+            if (rc) return rc;
+        }
         if (e & DERR_NAN) return set_err(c, PE_B200_ERR_NAN, "non-finite body state after step");
         if (e & DERR_TIMEOUT) return set_err(c, PE_B200_ERR_TIMEOUT, "device wait timed out");
         return set_err(c, PE_B200_ERR_CAPACITY, "device capacity exceeded");
@@ -1006,7 +1010,13 @@ int pe_b200_selftest_timeout(pe_b200_ctx *h, int64_t polls) {
     if (rc) return rc;
     rc = selftest_timeout(c, polls);
     if (rc) return rc;
-    return check_device_errors(c);
+    rc = check_device_errors(c);
+    if (rc != PE_B200_ERR_TIMEOUT) return rc;
+    int32_t left = 0;
+    const int brc = selftest_barriers(c, &left);
+    if (brc) return brc;
+    if (left) return set_err(c, PE_B200_ERR_CUDA, "arrivals left in a grid barrier after a timeout");
+    return rc;
 }
 
 int64_t pe_b200_kernel_launches(const pe_b200_ctx *h) {

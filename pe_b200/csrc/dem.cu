@@ -864,6 +864,7 @@ __global__ void __launch_bounds__(128) k_dem_contacts(DemArgs<VT> a0) {
     // launched early behind the rebuild kernel: nothing is read before it has finished
     pdl_wait();
     pdl_trigger();
+    if (timed_out(a0.err)) return;   // the rebuild may have left its lists half written
     const bool rebuilt = a0.nl_flags[4] != 0;
     const DemArgs<VT> a = list_view(a0);
     contacts_loop<VT, HERTZ, ONE, SPLIT, TRACKQ>(a, rebuilt, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
@@ -884,8 +885,10 @@ __global__ void __launch_bounds__(kRbBlock, MINB)
     pdl_wait();
     const bool rebuilt = ra.flags[0] != 0;
     if (rebuilt) {
-        if (!rebuild_stages(ra)) return;
-        if (!grid_sync(ra.bar, ra.err)) return;
+        if (!rebuild_stages(ra) || !grid_sync(ra.bar, ra.err)) {
+            ra.flags[0] = 1;   // a wait ran out: the lists are not complete
+            return;
+        }
     } else if (blockIdx.x == 0 && threadIdx.x == 0) {
         ra.flags[4] = 0;   // the integration reads the current state
     }
@@ -1005,17 +1008,20 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_dem_move(DemArgs<VT> a0) {
 // The barrier between two steps of k_list_steps, which also tells every block whether some block's
 // spheres asked for a rebuild: barrier number b uses word b % 3 (arrivals in the low half, requests
 // in the high half), one release-add and an acquire poll per block.  The word of barrier b - 2, which
-// every block has passed, is cleared for barrier b + 1.  Bounded: false when a wait gave up.
+// every block has passed, is cleared for barrier b + 1.  Bounded: false when a wait gave up, and (words[3]
+// then holds kGaveUp, and so does b) in the launches queued behind it.
 __device__ __forceinline__ bool steps_sync(unsigned int *words, unsigned int b, bool ask, bool *asked,
                                            int32_t *err) {
     __shared__ unsigned int s_v;
     const bool any = __syncthreads_or(ask ? 1 : 0) != 0;
     if (threadIdx.x == 0) {
         if (blockIdx.x == 0) atomicExch(words + (b + 1u) % 3u, 0u);
-        unsigned int *w = words + b % 3u, v;
-        asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(w), "r"(any ? 0x10001u : 1u) : "memory");
+        unsigned int *w = words + b % 3u, v = 0xffffffffu;
+        const bool meet = !(b & kGaveUp);
+        if (meet)
+            asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(w), "r"(any ? 0x10001u : 1u) : "memory");
         unsigned long long spins = 0;
-        for (;;) {
+        while (meet) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(w) : "memory");
             if ((v & 0xffffu) >= gridDim.x) break;
             if (++spins > 4096) __nanosleep(64);
@@ -1072,6 +1078,13 @@ __global__ void __launch_bounds__(kRbBlock, sizeof(VT) == 4 ? 3 : 2)
         marked = da.act[t + 1] > da.act[t];
         inverse_mass<T>(pi.w, ONE ? da.m0 : da.mats[tagi & 0xffffu], im, ii);
     };
+    // a wait ran out: the next step starts with a rebuild (the lists may be half written, and the
+    // path lengths since the last one are lost)
+    auto give_up = [&]() {
+        if (in) da.disp[t] = da.half_skin;
+        da.nl_flags[0] = 1;
+        if (threadIdx.x == 0) words[3] = kGaveUp;
+    };
     if (!rebuild) own(da.pr, da.vw, da.tag);
     for (int s = 0; s < steps; ++s) {
         const BodyBuf &from = (s & 1) ? other : mine, &to = (s & 1) ? mine : other;
@@ -1083,8 +1096,7 @@ __global__ void __launch_bounds__(kRbBlock, sizeof(VT) == 4 ? 3 : 2)
         if (rebuild) {
             ra.cur.pr = from.pr;
             ra.cur.vw = from.vw;
-            if (!rebuild_stages(ra)) return;
-            if (!grid_sync(ra.bar, ra.err)) return;
+            if (!rebuild_stages(ra) || !grid_sync(ra.bar, ra.err)) return give_up();
             a.pr = da.alt_pr;
             a.vw = da.alt_vw;
             a.tag = da.alt_tag;
@@ -1117,7 +1129,7 @@ __global__ void __launch_bounds__(kRbBlock, sizeof(VT) == 4 ? 3 : 2)
             moved = !(disp < a.half_skin);   // also catches NaN
         }
         // after an overflow every step rebuilds until the host has grown the list buffer
-        if (!steps_sync(words, base + (unsigned int)s, moved || !fits, &rebuild, ra.err)) return;
+        if (!steps_sync(words, base + (unsigned int)s, moved || !fits, &rebuild, ra.err)) return give_up();
     }
     if (in) da.disp[t] = disp;
     if (t == 0) {

@@ -479,7 +479,13 @@ const int2 *nbgs_ids_ptr(Ctx *c);
 // validate.cu: host checks of the device state; each adds the problems it finds to *bad
 int validate_coloring(Ctx *c, int64_t *bad);
 int validate_lists(Ctx *c, int64_t *bad);
+// runs a bounded wait out, leaving arrivals in the grid barriers as a block that gave up does;
+// selftest_barriers then counts the barriers that still hold any
 int selftest_timeout(Ctx *c, int64_t polls);
+int selftest_barriers(Ctx *c, int32_t *left);
+// the context's grid barriers as new, and the grid counts of the current state made again (they may
+// hold those of a step that ended early); the stream must be idle
+int reset_barriers(Ctx *c);
 void nbgs_free(Ctx *c);
 void nbgs_graph_free(Ctx *c);   // the captured hard-contact graphs
 
@@ -686,7 +692,14 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Grid-wide barrier for cooperative launches, with a bounded wait: a block that waits longer
 // than ~2 s records DERR_TIMEOUT and every thread of it sees false.  bar[0] counts arrivals,
 // bar[1] is the generation; both start at 0 and are left consistent after a completed barrier.
+// A wait that ran out leaves arrivals behind and marks bar[0] with kGaveUp: the launches queued behind
+// it end at their first barrier, until the host clears the words as it reports the timeout
+// (reset_barriers).
 constexpr unsigned long long kSpinLimit = 1ull << 24;  // polls of ~100 ns each
+constexpr unsigned int kGaveUp = 0x80000000u;
+__device__ __forceinline__ bool timed_out(const int32_t *err) {
+    return (*(const volatile int32_t *)err & DERR_TIMEOUT) != 0;
+}
 __device__ __forceinline__ bool grid_sync(unsigned int *bar, int32_t *err) {
     __shared__ int s_ok;
     __syncthreads();
@@ -696,7 +709,9 @@ __device__ __forceinline__ bool grid_sync(unsigned int *bar, int32_t *err) {
         __threadfence();
         const unsigned int arrived = atomicAdd(bar, 1u);
         int ok = 1;
-        if (arrived == gridDim.x - 1) {
+        if (arrived & kGaveUp) {
+            ok = 0;
+        } else if (arrived == gridDim.x - 1) {
             atomicExch(bar, 0u);
             __threadfence();
             atomicAdd(bar + 1, 1u);
@@ -708,6 +723,7 @@ __device__ __forceinline__ bool grid_sync(unsigned int *bar, int32_t *err) {
                 if (++spins > 4096) __nanosleep(128);
                 if (spins > kSpinLimit) {
                     ok = 0;
+                    atomicOr(bar, kGaveUp);
                     atomicOr(err, DERR_TIMEOUT);
                     break;
                 }

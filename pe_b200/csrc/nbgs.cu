@@ -737,8 +737,10 @@ __global__ void k_color_pos(const int32_t *ncp, const int32_t *dd, const int32_t
 template <typename T, bool GEN>
 __global__ void k_cache(const int32_t *ncp, const int32_t *dd, int64_t cap, Raw<T> raw,
                         const int32_t *pos, const int32_t *color, const uint64_t *used,
-                        const int32_t *adj_start, int32_t *adj, BodyV<T> bv, int64_t nb, Cache<T> cc) {
+                        const int32_t *adj_start, int32_t *adj, BodyV<T> bv, int64_t nb, Cache<T> cc,
+                        const int32_t *err) {
     if (dd[kDdAbort]) return;
+    if (adj && timed_out(err)) adj = nullptr;   // the degrees may not be summed; nothing follows them
     const int64_t nc = *ncp;
     GRID_STRIDE(c, nc) {
     const int64_t k = pos[c];
@@ -1814,7 +1816,8 @@ __global__ void __launch_bounds__(kFlowBlk, sizeof(T) == 4 ? 5 : 3)
                   int track_last, unsigned long long *delta, int32_t *err) {
     constexpr int N = FlowRec<T>::N;
     if (!sweeps_gate(dd, gate)) return;
-    if (*(volatile int32_t *)err & DERR_COLORS) return;   // no valid colouring to follow
+    // no valid colouring to follow, or one that ended early
+    if (__syncthreads_or(*(volatile int32_t *)err & (DERR_COLORS | DERR_TIMEOUT))) return;
     __shared__ int32_t cs[kMaxColors + 1], goff[kMaxColors + 1];
     __shared__ int s_size;
     const int ncolors = dd[kDdNcolors];
@@ -2952,10 +2955,10 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
         prof_begin(c, ST_CACHE);
         // 4. contact cache in colour-sorted order
         if constexpr (std::is_same<VT, double>::value) {
-            if (gen) k_cache<VT, true><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
-            else k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
+            if (gen) k_cache<VT, true><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc, c->d_err);
+            else k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc, c->d_err);
         } else {
-            k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc);
+            k_cache<VT, false><<<cgrid, kBlk, 0, c->stream>>>(ncp, dd, cap, raw, nb.order, nb.color, nb.used, nb.body_cnt, flow_adj, bv, n, cc, c->d_err);
         }
         PEB_LAUNCHED(c);
         prof_end(c, ST_CACHE);

@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(kRbBlock) k_rebuild(RebuildArgs<VT> a) {
         pdl_trigger();
         return;
     }
-    rebuild_stages(a);
+    if (!rebuild_stages(a)) a.flags[0] = 1;   // a wait ran out: the lists are not complete
 }
 
 template <typename VT>

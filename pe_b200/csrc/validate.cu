@@ -16,8 +16,22 @@ namespace {
 
 // Waits for a flag nothing sets, with the bounded poll of the grid barriers: after `polls`
 // polls it records DERR_TIMEOUT and returns, leaving the context usable.
-__global__ void k_wait_never(const unsigned int *flag, unsigned long long polls, int32_t *err) {
+// First it arrives at the context's grid barriers (null: not there), which nothing completes, and
+// marks them as a block that gives up does.
+__global__ void k_wait_never(const unsigned int *flag, unsigned long long polls, int32_t *err,
+                             unsigned int *bar0, unsigned int *bar1, unsigned int *bar2,
+                             unsigned int *steps) {
     if (threadIdx.x != 0) return;
+    unsigned int *bars[] = {bar0, bar1, bar2};
+    for (unsigned int *b : bars)
+        if (b) {
+            atomicAdd(b, 1u);
+            atomicOr(b, kGaveUp);
+        }
+    if (steps) {
+        atomicAdd(steps + (steps[3] & 3u), 0x10001u);
+        steps[3] = kGaveUp;
+    }
     unsigned long long spins = 0;
     for (;;) {
         unsigned int v;
@@ -81,13 +95,38 @@ int selftest_timeout(Ctx *c, int64_t polls) {
     PEB_CUDA(c, dmalloc(c, &flag, sizeof(unsigned int)));
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(unsigned int), c->stream);
     if (e == cudaSuccess) {
-        k_wait_never<<<1, 32, 0, c->stream>>>(flag, (unsigned long long)polls, c->d_err);
+        k_wait_never<<<1, 32, 0, c->stream>>>(flag, (unsigned long long)polls, c->d_err, c->gs_bar,
+                                              c->nl.rb_bar, c->nb.bar2, c->nl.steps_bar);
         e = cudaGetLastError();
         c->launches++;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     dfree(c, flag);
     if (e != cudaSuccess) return cuda_err(c, e, "timeout self-test");
+    return PE_B200_OK;
+}
+
+int reset_barriers(Ctx *c) {
+    unsigned int *bars[] = {c->gs_bar, c->nl.rb_bar, c->nb.bar2};
+    for (unsigned int *b : bars)
+        if (b) PEB_CUDA(c, cudaMemsetAsync(b, 0, 2 * sizeof(unsigned int), c->stream));
+    if (c->nl.steps_bar)
+        PEB_CUDA(c, cudaMemsetAsync(c->nl.steps_bar, 0, 4 * sizeof(unsigned int), c->stream));
+    c->binned = false;
+    return PE_B200_OK;
+}
+
+int selftest_barriers(Ctx *c, int32_t *left) {
+    *left = 0;
+    unsigned int *bars[] = {c->gs_bar, c->nl.rb_bar, c->nb.bar2, c->nl.steps_bar};
+    for (int k = 0; k < 4; ++k) {
+        if (!bars[k]) continue;
+        unsigned int w[4] = {0, 0, 0, 0};
+        PEB_CUDA(c, cudaMemcpyAsync(w, bars[k], (k < 3 ? 1 : 4) * sizeof(unsigned int),
+                                    cudaMemcpyDeviceToHost, c->stream));
+        PEB_CUDA(c, cudaStreamSynchronize(c->stream));
+        *left += (w[0] | w[1] | w[2] | w[3]) != 0u ? 1 : 0;
+    }
     return PE_B200_OK;
 }
 
