@@ -607,6 +607,8 @@ def our_arm(args):
         form = (tuning or {}).get("dem_split", 0)
         kname = {0: "the list step: k_rebuild_contacts (rebuild check, marked spheres' forces), "
                     "then k_dem_move (integration of every sphere)",
+                 -1: "the list step in the form the library picks: overlapped at this size (as form "
+                     "2), many steps in one kernel for small scenes",
                  1: "the list step: k_rebuild (rebuild check), then k_dem_contacts (marked "
                     "spheres) on a second stream beside k_dem_move (the others)",
                  2: "the list step, overlapped: k_rebuild_contacts (rebuild check, marked "

@@ -417,7 +417,10 @@ int run_steps(Ctx *c, int32_t nsteps, double dt) {
         }
         return PE_B200_OK;
     }
-    if (c->p.solver == PE_B200_DEM && c->nl.enabled) dem_list_pick(c);
+    if (c->p.solver == PE_B200_DEM && c->nl.enabled) {
+        const int rc = dem_list_pick(c);
+        if (rc) return rc;
+    }
     if (c->p.solver == PE_B200_DEM && c->nl.enabled && !c->prof) {
         int rc = dem_list_graph_run(c, nsteps, dt, &k);
         if (rc) return rc;

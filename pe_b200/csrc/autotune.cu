@@ -9,11 +9,13 @@
 //                   one launch per stage instead (the same lists, entry for entry)
 //   skin            neighbour-list skin (cells are re-planned to 2 r_max + skin)
 //   dem_split       form of the list step: the contact forces before the integration, on a
-//                   second stream beside it, or overlapped with it on one stream (dem.cu)
+//                   second stream beside it, or overlapped with it on one stream (dem.cu); -1, a
+//                   new context's value: the library's choice, with many steps of a small scene
+//                   in one kernel
 // Each trial restores the state saved at entry, forces a list rebuild, runs a few untimed steps
 // (graph capture included), then times `trial` steps with CUDA events after forcing one more
 // rebuild, so a trial's time charges at least one rebuild per `trial` steps.  Coordinate
-// descent: skin first, then the force kernel's shape, then the rebuild grid.
+// descent: skin first, then the force kernel's shape, then the rebuild grid, then the form.
 #include <algorithm>
 #include <cmath>
 
@@ -71,12 +73,11 @@ int set_list_skin(Ctx *c, double skin) {
 int set_tuning(Ctx *c, const Tuning &t, double skin) {
     if (t.dem_variant < 0 || t.dem_variant >= dem_variant_count() || t.rebuild_per_sm < -1 ||
         t.nbgs_sweeps < 0 || t.nbgs_sweeps > 5 || t.dem_grid < 0 || t.dem_grid > 1 ||
-        t.dem_split < 0 || t.dem_split > 2)
+        t.dem_split < -1 || t.dem_split > 2)
         return set_err(c, PE_B200_ERR_ARG, "invalid tuning");
     // captured list-step graphs bake the form in; the new form's first step runs outside a
     // capture (the split form creates its second stream there)
-    if (c->form_auto || t.dem_split != c->tune.dem_split) {
-        c->form_auto = false;   // the caller's form from here on
+    if (t.dem_split != c->tune.dem_split) {
         c->epoch++;
         c->nl.warm = false;
     }
@@ -125,6 +126,11 @@ int autotune(Ctx *c, double dt, int32_t trial, pe_b200_tuning *out) {
         if (!r) r = set_tuning(c, t, skin);
         if (!r) r = dem_list_request_rebuild(c);
         if (!r) r = run_steps(c, warm, dt);
+        if (!r && t.dem_split < 0) {
+            // the library picks by the list entries of those steps; a change of form is captured here
+            PEB_CUDA(c, cudaStreamSynchronize(c->stream));
+            r = run_steps(c, warm, dt);
+        }
         if (!r) r = dem_list_request_rebuild(c);
         if (r) return r;
         PEB_CUDA(c, cudaEventRecord(e0, c->stream));
@@ -167,16 +173,21 @@ int autotune(Ctx *c, double dt, int32_t trial, pe_b200_tuning *out) {
         rc = consider(t, best_skin);
     }
     const int32_t split0 = best.dem_split;
-    for (int32_t f = 0; f <= 2; ++f) {
+    for (int32_t f = -1; f <= 2; ++f) {
         if (rc || f == split0) continue;
         Tuning t = best;
         t.dem_split = f;
         rc = consider(t, best_skin);
     }
-    // leave the state as it was at entry, with the winning shapes
-    if (!rc) rc = copy_bodies(c, c->cur, snap);
-    if (!rc) rc = set_tuning(c, best, best_skin);
-    if (!rc) rc = dem_list_request_rebuild(c);
+    // leave the state as it was at entry, with the winning shapes (after a failure, the caller's)
+    if (rc) {
+        best = t0;
+        best_skin = skin0;
+    }
+    int rc2 = copy_bodies(c, c->cur, snap);
+    if (!rc2) rc2 = set_tuning(c, best, best_skin);
+    if (!rc2) rc2 = dem_list_request_rebuild(c);
+    if (!rc) rc = rc2;
     cudaStreamSynchronize(c->stream);
     c->prof = prof0;
     cudaEventDestroy(e0);

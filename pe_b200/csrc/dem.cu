@@ -1417,8 +1417,8 @@ bool split_streams(Ctx *c) {
     return true;
 }
 
-// the form of the list step (Tuning.dem_split), the caller's or the one picked for the scene
-int list_form(const Ctx *c) { return c->form_auto ? c->nl.form : c->tune.dem_split; }
+// the form of the list step, the caller's (Tuning.dem_split) or the one picked for the scene
+int list_form(const Ctx *c) { return c->tune.dem_split < 0 ? c->nl.form : c->tune.dem_split; }
 
 // contacts_done: the fused rebuild-and-contacts kernel has run (1: it stored the marked spheres'
 // forces; 2: the overlapped form, it integrates them too)
@@ -1863,11 +1863,12 @@ void graph_key(const Ctx *c, const void *key[12]) {
 }
 
 // Whether the library runs `steps` consecutive list steps of this scene as one kernel: a linear-law
-// scene without orientations, no form set by the caller, every sphere a thread of the resident
-// grid, and an even count (the two state buffers end where they began).
+// scene without orientations, no form set by the caller, cooperative launches not turned off, every
+// sphere a thread of the resident grid, and an even count (the two state buffers end where they
+// began).
 bool steps_fit_kernel(const Ctx *c, int32_t steps) {
-    return c->form_auto && !c->nl.steps_off && !c->nl.coop_disabled && !c->prof && (steps & 1) == 0 &&
-           !c->p.track_orientation && c->p.force_model == 0 && c->n <= kStepsMax;
+    return c->tune.dem_split < 0 && c->tune.rebuild_per_sm >= 0 && !c->nl.steps_off &&
+           !c->nl.coop_disabled && !c->prof && (steps & 1) == 0 && !c->p.track_orientation && c->p.force_model == 0 && c->n <= kStepsMax;
 }
 
 template <typename VT>
@@ -1973,18 +1974,21 @@ int capture_steps(Ctx *c, int32_t steps, double dt) {
 // 97,336 23.8 / 22.5, 704,969 108 / 100; mixed mostly apart 400,000 10.5 / 10.3, 700,000 16.1 / 15.6,
 // 200,000 8.3 / 10.0; mixed in contact 29,791 11.9 / 10.8, 195,112 27.7 / 24.4, 1,048,576 134 / 107,
 // 8,000 10.3 / 10.5.  Batches of scenes stay plain (1.0M spheres in 64: 42.5 / 46.3).
-void dem_list_pick(Ctx *c) {
-    if (!c->form_auto) return;
+int dem_list_pick(Ctx *c) {
+    if (c->tune.dem_split >= 0 || c->n == 0) return PE_B200_OK;
+    const int rc = list_capacity_check(c);   // the entries, if a read-back has come since
+    if (rc) return rc;
     const bool one = c->nscenes == 1 && c->mats.size() == 1 && !c->p.track_orientation &&
                      c->p.force_model == 0;
     const bool dense = c->nl.entries >= 2 * c->n;   // at the rebuild last read back
     const bool fp64 = c->p.precision == PE_B200_FP64;
     const bool over = dense ? fp64 || c->n >= 25000 : c->n >= (fp64 ? 100000 : 400000);
     const int form = one && over ? 2 : 0;
-    if (form == c->nl.form) return;
+    if (form == c->nl.form) return PE_B200_OK;
     c->nl.form = form;
     c->epoch++;             // captured steps bake the form in
     c->nl.warm = false;     // and its first step runs outside a capture
+    return PE_B200_OK;
 }
 
 int dem_list_step(Ctx *c, double dt) {

@@ -196,7 +196,7 @@ struct ListBuf {
     bool warm = false;          // a list step has run since the buffers were (re)allocated
     int since_check = 1 << 20;  // steps since the last queued read-back of flags
     int64_t entries = 0;        // list entries at the rebuild last read back
-    int form = 0;               // the step's form when the library picks it (dem_list_pick)
+    int form = 0;               // the step's form while tuning.dem_split is -1 (dem_list_pick)
 };
 
 // launch shapes of the DEM list step, picked by pe_b200_autotune (autotune.cu)
@@ -206,7 +206,7 @@ struct Tuning {
     int32_t nbgs_sweeps = 0;    // 0 automatic, 1 one cluster, 2 cooperative grid, 3 per colour,
                                 // 4 one block, 5 bodies in one cluster's shared memory
     int32_t dem_grid = 0;       // grid step: 0 sorted FP32 candidate copy, 1 FP64 records only
-    int32_t dem_split = 0;      // list step: 1 the marked spheres on a second stream (dem.cu)
+    int32_t dem_split = -1;     // form of the list step (dem.cu); -1: dem_list_pick's
 };
 
 // a captured CUDA graph of `steps` DEM list steps (dem.cu); valid while the buffers it was
@@ -313,7 +313,6 @@ struct Ctx {
     MBoxBuf mb;
     AdjState adj;
     Tuning tune;
-    bool form_auto = true;          // no tuning was set: the library picks the list step's form
     StepGraph sg;
     void *stage = nullptr;          // host-layout staging for uploads and downloads (transfer.cu)
     size_t stage_bytes = 0;
@@ -419,7 +418,7 @@ void dem_list_free(Ctx *c);
 int dem_list_request_rebuild(Ctx *c);
 int dem_list_rebuild_persistent(Ctx *c);
 int dem_list_step(Ctx *c, double dt);
-void dem_list_pick(Ctx *c);
+int dem_list_pick(Ctx *c);
 // runs whole graph replays of c->graph_steps list steps while they fit in nsteps; *done
 // receives the steps run (0 when graphs are off or not possible)
 int dem_list_graph_run(Ctx *c, int32_t nsteps, double dt, int32_t *done);

@@ -262,8 +262,12 @@ class Engine:
         return {k: getattr(t, k) for k, _ in _abi.Tuning._fields_}
 
     def set_tuning(self, dem_variant: int = 0, rebuild_per_sm: int = 0, skin: float = 0.0,
-                   nbgs_sweeps: int = 0, dem_grid: int = 0, dem_split: int = 0):
-        """skin <= 0 keeps the current skin."""
+                   nbgs_sweeps: int = 0, dem_grid: int = 0, dem_split: int = 0,
+                   ms_per_step=None, variants=None):
+        """Sets every field; skin <= 0 keeps the current skin.  dem_split -1, a new context's value,
+        lets the library pick the list step's form.  To change one field and keep the others start
+        from tuning(): ``e.set_tuning(**dict(e.tuning(), dem_grid=1))`` (the outputs it returns,
+        ms_per_step and variants, are ignored here)."""
         if skin <= 0:
             skin = self.tuning()["skin"]
         t = _abi.Tuning(dem_variant=dem_variant, rebuild_per_sm=rebuild_per_sm, skin=skin,
