@@ -33,6 +33,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "list_form.h"
 #include "near.cuh"
 #include "rebuild.cuh"
 
@@ -1965,25 +1966,16 @@ int capture_steps(Ctx *c, int32_t steps, double dt) {
 
 }  // namespace
 
-// Picks the list step's form for a caller that did not: the overlapped one (2) or the plain one
-// (0); all give the same results.  Overlapping pays once the contact kernel, which then
-// integrates its spheres too, is long enough beside the integration of the others, and costs a
-// longer start (its release and the last block's wait).  One scene of one material, us per step
-// (plain / overlapped): FP64 mostly apart 100,000 spheres 6.6 / 6.3, 200,000 9.2 / 7.7, 700,000 21.7
-// / 19.1, 30,000 5.2 / 5.9; FP64 in contact (2 list entries a sphere or more) 2,197 11.5 / 10.9,
-// 97,336 23.8 / 22.5, 704,969 108 / 100; mixed mostly apart 400,000 10.5 / 10.3, 700,000 16.1 / 15.6,
-// 200,000 8.3 / 10.0; mixed in contact 29,791 11.9 / 10.8, 195,112 27.7 / 24.4, 1,048,576 134 / 107,
-// 8,000 10.3 / 10.5.  Batches of scenes stay plain (1.0M spheres in 64: 42.5 / 46.3).
+// Picks the list step's form for a caller that did not (list_form.h), by the entries of the rebuild
+// last read back.
 int dem_list_pick(Ctx *c) {
     if (c->tune.dem_split >= 0 || c->n == 0) return PE_B200_OK;
     const int rc = list_capacity_check(c);   // the entries, if a read-back has come since
     if (rc) return rc;
     const bool one = c->nscenes == 1 && c->mats.size() == 1 && !c->p.track_orientation &&
                      c->p.force_model == 0;
-    const bool dense = c->nl.entries >= 2 * c->n;   // at the rebuild last read back
-    const bool fp64 = c->p.precision == PE_B200_FP64;
-    const bool over = dense ? fp64 || c->n >= 25000 : c->n >= (fp64 ? 100000 : 400000);
-    const int form = one && over ? 2 : 0;
+    c->nl.dense = list_dense(c->nl.dense, c->n, c->nl.entries);
+    const int form = list_form_rule(one, c->p.precision == PE_B200_FP64, c->n, c->nl.dense);
     if (form == c->nl.form) return PE_B200_OK;
     c->nl.form = form;
     c->epoch++;             // captured steps bake the form in

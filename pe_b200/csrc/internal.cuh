@@ -196,6 +196,7 @@ struct ListBuf {
     bool warm = false;          // a list step has run since the buffers were (re)allocated
     int since_check = 1 << 20;  // steps since the last queued read-back of flags
     int64_t entries = 0;        // list entries at the rebuild last read back
+    bool dense = false;         // and whether they make the scene one in contact (list_form.h)
     int form = 0;               // the step's form while tuning.dem_split is -1 (dem_list_pick)
 };
 
