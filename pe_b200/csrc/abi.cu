@@ -55,7 +55,12 @@ cudaError_t dmalloc_bytes(Ctx *c, void **p, size_t bytes) {
     cudaMemPool_t pool = nullptr;
     cudaError_t e = lib_pool(c->device, &pool);
     if (e != cudaSuccess) return e;
-    return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, c->stream);
+    e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, c->stream);
+    if (e == cudaErrorMemoryAllocation && nbgs_flow_free(c)) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, c->stream);
+    }
+    return e;
 }
 
 void dfree(Ctx *c, void *p) {

@@ -104,6 +104,8 @@ struct NbgsBuf {
     unsigned int *bar2 = nullptr;             // grid barrier of the colouring rounds
     int32_t *slot_of = nullptr;               // per body: -1, or its claim in the compact sweep
     bool flow_off = false;                    // the sweep form without barriers cannot be launched
+    void *flow = nullptr;                     // its places and mailboxes, for flow_cap contacts
+    int64_t flow_cap = 0;
     bool compact_off = false;                 // the compact sweep form cannot be launched
     bool staged_off = false;                  // nor the grid form with staged contacts
     bool on_device = false;                   // the last step's counts are only on the device
@@ -347,6 +349,8 @@ enum : int32_t {
 // contexts free (abi.cu): a new context reuses the memory of the ones before it instead of
 // mapping fresh pages.  dmalloc allocates on the context's stream, dfree frees there (nullptr
 // allowed).
+// allocates on the context's stream; when the memory is short, after giving back what the context can
+// do without (nbgs_flow_free)
 cudaError_t dmalloc_bytes(Ctx *c, void **p, size_t bytes);
 void dfree(Ctx *c, void *p);
 template <typename T>
@@ -488,6 +492,8 @@ int selftest_barriers(Ctx *c, int32_t *left);
 int reset_barriers(Ctx *c);
 void nbgs_free(Ctx *c);
 void nbgs_graph_free(Ctx *c);   // the captured hard-contact graphs
+// gives back the buffers of the sweeps without barriers, which then stay off; false: there are none
+bool nbgs_flow_free(Ctx *c);
 
 // ------------------------------------------------------------------------------------------
 // device helpers

@@ -745,9 +745,10 @@ __global__ void k_cache(const int32_t *ncp, const int32_t *dd, int64_t cap, Raw<
     GRID_STRIDE(c, nc) {
     const int64_t k = pos[c];
     const int32_t b1 = raw.b1[c], b2 = raw.b2[c];
-    // the contact's place among each of its bodies' contacts in colour order, and their number
-    // (a body has one contact per colour of its mask)
-    {
+    // for the sweeps without barriers: the contact's place among each of its bodies' contacts in
+    // colour order, and their number (a body has one contact per colour of its mask); the bodies'
+    // contacts in that order, and empty mailboxes
+    if (adj) {
         constexpr int W = GEN ? 4 : 1;
         const int col = color[c];
         auto place = [&](int32_t b, int &s, int &d) {
@@ -765,14 +766,11 @@ __global__ void k_cache(const int32_t *ncp, const int32_t *dd, int64_t cap, Raw<
         place(b1, sq.x, sq.y);
         place(b2, sq.z, sq.w);
         cc.seq[k] = sq;
-        if (adj) {
-            // the bodies' contacts in colour order, and empty mailboxes
-            if (sq.x < sq.y) adj[adj_start[b1] + sq.x] = (int32_t)(2 * k);
-            if (sq.z < sq.w) adj[adj_start[b2] + sq.z] = (int32_t)(2 * k + 1);
+        if (sq.x < sq.y) adj[adj_start[b1] + sq.x] = (int32_t)(2 * k);
+        if (sq.z < sq.w) adj[adj_start[b2] + sq.z] = (int32_t)(2 * k + 1);
 #pragma unroll
-            for (int q = 0; q < (int)sizeof(T); ++q)   // FlowRec<T>::N vectors for each side
-                cc.mail[2 * ((q >> 1) * cap + k) + (q & 1)] = make_ulonglong2(0ull, 0ull);
-        }
+        for (int q = 0; q < (int)sizeof(T); ++q)   // FlowRec<T>::N vectors for each side
+            cc.mail[2 * ((q >> 1) * cap + k) + (q & 1)] = make_ulonglong2(0ull, 0ull);
     }
     const V3<T> r1 = ld3c(raw.r1, c, cap), r2 = ld3c(raw.r2, c, cap), n = ld3c(raw.n, c, cap);
     V3<T> t;
@@ -2063,8 +2061,8 @@ int nbgs_alloc(Ctx *c, int64_t cap) {
         b.color = nullptr;
         dfree(c, b.body_adj);
         b.body_adj = nullptr;
-        // raw: 2 int + 11 T; cache: 6 int + (kRec + 3) x 4 T, and 16 T of mailboxes (per contact)
-        const size_t bytes = (size_t)cap * (8 * sizeof(int32_t) + (11 + 4 * (kRec + 3) + 16) * es) + 64 * 256;
+        // raw: 2 int + 11 T; cache: 2 int + (kRec + 3) x 4 T  (per contact)
+        const size_t bytes = (size_t)cap * (4 * sizeof(int32_t) + (11 + 4 * (kRec + 3)) * es) + 64 * 256;
         PEB_CUDA(c, dmalloc(c, &b.cache, bytes));
         PEB_CUDA(c, dmalloc(c, &b.order, (size_t)cap * sizeof(int32_t)));
         PEB_CUDA(c, dmalloc(c, &b.color, (size_t)cap * sizeof(int32_t)));
@@ -2147,8 +2145,8 @@ void layout(Ctx *c, Raw<T> &raw, Cache<T> &cc, BodyV<T> &bv) {
     cc.rec = (T4<T> *)take(kRec * cap * sizeof(T4<T>));
     cc.p = (T4<T> *)take(cap * sizeof(T4<T>));
     cc.dc = (T4<T> *)take(2 * cap * sizeof(T4<T>));
-    cc.seq = (int4 *)take(cap * sizeof(int4));
-    cc.mail = (ulonglong2 *)take(cap * 16 * sizeof(T));
+    cc.seq = nullptr;    // flow_buffers
+    cc.mail = nullptr;
     const int64_t n = b.nbod;
     T4<T> *v = (T4<T> *)b.vel;
     bv.vr = v;
@@ -2162,6 +2160,32 @@ void layout(Ctx *c, Raw<T> &raw, Cache<T> &cc, BodyV<T> &bv) {
     } else {
         bv.ia = bv.ib = bv.ic = nullptr;
     }
+}
+
+// The buffers of the sweeps without barriers, for the contact capacity: a place (4 int) and mailboxes
+// (16 T) per contact.  They are apart from the contact cache, so that a context whose sweeps take
+// another form, or a scene that leaves no room for them, does without.  true: they are there.
+bool flow_reserve(Ctx *c) {
+    NbgsBuf &b = c->nb;
+    if (b.flow_off || c->tune.nbgs_sweeps != 0) return false;
+    if (b.flow && b.flow_cap >= b.cap) return true;
+    if (b.flow) nbgs_graph_free(c);
+    dfree(c, b.flow);
+    b.flow = nullptr;
+    const size_t es = (c->p.precision == PE_B200_FP64) ? 8 : 4;
+    if (dmalloc(c, &b.flow, (size_t)b.cap * (4 * sizeof(int32_t) + 16 * es)) != cudaSuccess) {
+        cudaGetLastError();
+        b.flow = nullptr;
+        b.flow_off = true;
+        return false;
+    }
+    b.flow_cap = b.cap;
+    return true;
+}
+template <typename T>
+void flow_buffers(Ctx *c, Cache<T> &cc) {
+    cc.mail = (ulonglong2 *)c->nb.flow;
+    cc.seq = (int4 *)(cc.mail + c->nb.flow_cap * (int64_t)sizeof(T));
 }
 
 // the sweep kernels of relaxation model m (pe's RelaxationModel 0-5)
@@ -2863,8 +2887,11 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     // (93 contacts at the end) 3260 / 3152, 2x4x4 (145) 3373 / 3501, 6x6x6 6242 / 7910.
     const int64_t flow_min = !gen ? kCompactMax
                              : c->p.relaxation_model == PE_B200_INELASTIC_FRICTIONLESS ? 1100 : 96;
-    int32_t *flow_adj = c->tune.nbgs_sweeps == 0 && !nb.flow_off && !few && (queued || nc > flow_min)
-                            ? nb.body_adj : nullptr;
+    int32_t *flow_adj = nullptr;
+    if (any && !few && (queued || nc > flow_min) && flow_reserve(c)) {
+        flow_adj = nb.body_adj;
+        flow_buffers<VT>(c, cc);
+    }
     if (any) {
         prof_begin(c, ST_COLOR);
         const size_t masks = (size_t)nbod * (gen ? 4 : 1) * sizeof(uint64_t);
@@ -3152,10 +3179,24 @@ void nbgs_free(Ctx *c) {
     dfree(c, b.rem);
     dfree(c, b.bar2);
     dfree(c, b.slot_of);
+    dfree(c, b.flow);
     if (b.color_start) cudaFreeHost(b.color_start);
     if (b.h_dd) cudaFreeHost(b.h_dd);
     nbgs_graph_free(c);
     b = NbgsBuf();
+}
+
+bool nbgs_flow_free(Ctx *c) {
+    NbgsBuf &b = c->nb;
+    if (!b.flow) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    nbgs_graph_free(c);
+    dfree(c, b.flow);
+    b.flow = nullptr;
+    b.flow_cap = 0;
+    b.flow_off = true;
+    return cudaStreamSynchronize(c->stream) == cudaSuccess;
 }
 
 void nbgs_graph_free(Ctx *c) {
@@ -3216,6 +3257,8 @@ int nbgs_graph_run(Ctx *c, int32_t nsteps, double dt, int32_t *ran) {
         if (!s.exec || (lru->exec && s.used < lru->used)) lru = &s;
     }
     if (!hit) {
+        // nothing is allocated inside a capture
+        if (!nb.plan_none && !nb.plan_few) flow_reserve(c);
         hit = lru;
         if (hit->exec) cudaGraphExecDestroy(hit->exec);
         hit->exec = nullptr;
