@@ -56,8 +56,10 @@ cudaError_t dmalloc_bytes(Ctx *c, void **p, size_t bytes) {
     cudaError_t e = lib_pool(c->device, &pool);
     if (e != cudaSuccess) return e;
     e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, c->stream);
-    if (e == cudaErrorMemoryAllocation && nbgs_flow_free(c)) {
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
+        const bool flow = nbgs_flow_free(c), adj = adjoint_spare_free(c);
+        if (!flow && !adj) return e;
         e = cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pool, c->stream);
     }
     return e;

@@ -357,6 +357,21 @@ void adjoint_free(Ctx *c) {
     c->adj.nsteps = 0;
 }
 
+bool adjoint_spare_free(Ctx *c) {
+    AdjState &A = c->adj;
+    const bool search = A.search && A.busy < 2, seg = !A.seg.empty() && A.busy < 1;
+    if (search) {
+        dfree(c, A.search);
+        A.search = nullptr;
+        A.search_bytes = 0;
+    }
+    if (seg) {
+        for (auto &b : A.seg) free_ckpt(c, b);
+        A.seg.clear();
+    }
+    return search || seg;
+}
+
 int adjoint_forward(Ctx *c, int32_t nsteps, double dt, int32_t every) {
     if (c->p.solver != PE_B200_DEM || c->p.precision != PE_B200_FP64 || c->p.track_orientation ||
         c->p.force_model != 0)
@@ -427,6 +442,7 @@ int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *g
     // the pre-step states of a segment after its checkpoint (the forward run's last segment may
     // be shorter than the interval)
     const int seglen = std::min(A.every, A.nsteps);
+    A.busy = 1;
     for (size_t k = A.seg.size(); k + 1 < (size_t)seglen && !rc; ++k) {
         BodyBuf b;
         rc = alloc_ckpt(c, b);
@@ -445,6 +461,7 @@ int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *g
         else cudaGetLastError();
     }
     const bool kept = keep && A.search_bytes >= per * seglen;
+    A.busy = 2;
     // the steps below run on the checkpoints' and the segment's buffers, and search into the kept
     // ones; the context's own state stays what it is
     const BodyBuf cur0 = c->cur, nxt0 = c->nxt;
@@ -532,6 +549,7 @@ int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *g
     c->near = near0;
     c->tune.dem_grid = grid0;
     c->binned = false;
+    A.busy = 0;
     if (!rc) {
         std::vector<double> hp(4 * (size_t)blocks);
         e = cudaMemcpyAsync(ox, l[cur_l], vb, cudaMemcpyDeviceToHost, c->stream);

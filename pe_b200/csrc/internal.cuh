@@ -232,6 +232,7 @@ struct AdjState {
     std::vector<BodyBuf> seg;    // pre-step states of the segment being reversed, after the first
     int32_t *search = nullptr;   // their sorts and candidate lists, while they are small enough
     int64_t search_bytes = 0;
+    int busy = 0;                // a backward pass runs on seg (1), and on search (2)
 };
 
 // stage timers (pe's profiling sections, e.g. DEMSolver.h:1159-1260): CUDA events around each
@@ -350,7 +351,7 @@ enum : int32_t {
 // mapping fresh pages.  dmalloc allocates on the context's stream, dfree frees there (nullptr
 // allowed).
 // allocates on the context's stream; when the memory is short, after giving back what the context can
-// do without (nbgs_flow_free)
+// do without (nbgs_flow_free, adjoint_spare_free)
 cudaError_t dmalloc_bytes(Ctx *c, void **p, size_t bytes);
 void dfree(Ctx *c, void *p);
 template <typename T>
@@ -451,6 +452,9 @@ int adjoint_forward(Ctx *c, int32_t nsteps, double dt, int32_t every);
 int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *gw, double *ox,
                      double *ov, double *ow, double *gpar);
 void adjoint_free(Ctx *c);
+// gives back the segment and search buffers kept for the next backward pass, but for those that a
+// running one uses; false: there are none
+bool adjoint_spare_free(Ctx *c);
 int nbgs_step(Ctx *c, double dt);
 int nbgs_run(Ctx *c, int32_t nsteps, double dt);   // nsteps steps (retries aborted queued ones)
 int find_contacts(Ctx *c, int64_t cap, int64_t *ids, double *geom, int64_t *n_out);
