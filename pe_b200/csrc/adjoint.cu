@@ -449,6 +449,9 @@ int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *g
         if (rc) free_ckpt(c, b);
         else A.seg.push_back(b);
     }
+    // what each step searches with, made here rather than by the first one, so that the kept lists can
+    // stand in (and before they take what memory there is)
+    if (!rc) rc = near_reserve(c);
     // the segment's sorts and candidate lists: per step the cell offsets, the order, the lists
     const int64_t nn = std::max<int64_t>(n, 1);
     const int64_t per = ((c->ncell + 2 + nn + (1 + kNear) * nn) * (int64_t)sizeof(int32_t) + 255) & ~(int64_t)255;
@@ -465,16 +468,9 @@ int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *g
     // the steps below run on the checkpoints' and the segment's buffers, and search into the kept
     // ones; the context's own state stays what it is
     const BodyBuf cur0 = c->cur, nxt0 = c->nxt;
-    int32_t *const sorted0 = c->sorted, *const start0 = c->cell_start, *near0 = c->near;
+    int32_t *const sorted0 = c->sorted, *const start0 = c->cell_start, *const near0 = c->near;
     const int32_t grid0 = c->tune.dem_grid;
     c->tune.dem_grid = 0;   // the form with candidate lists (both give the same states)
-    if (!rc && !c->posf) {
-        // allocated here rather than by the first step, so that the kept lists can stand in
-        e = dmalloc(c, &c->posf, (size_t)nn * sizeof(float4));
-        if (e == cudaSuccess) e = dmalloc(c, &c->near, (size_t)nn * (1 + kNear) * sizeof(int32_t));
-        if (e != cudaSuccess) rc = cuda_err(c, e, "adjoint buffers");
-        near0 = c->near;
-    }
     auto use = [&](int s) {   // the search buffers of the segment's s-th state
         if (!kept) return;
         int32_t *p = (int32_t *)((char *)A.search + per * s);

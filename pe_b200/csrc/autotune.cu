@@ -58,6 +58,7 @@ int set_list_skin(Ctx *c, double skin) {
     dfree(c, c->cell_count);
     dfree(c, c->cell_start);
     c->cell_count = c->cell_start = nullptr;
+    c->uploaded = false;   // until the new cells are there
     PEB_CUDA(c, dmalloc(c, &c->cell_count, ((size_t)c->ncell + 1) * sizeof(int32_t)));
     PEB_CUDA(c, dmalloc(c, &c->cell_start, ((size_t)c->ncell + 2) * sizeof(int32_t)));
     PEB_CUDA(c, cudaMemsetAsync(c->cell_count, 0, ((size_t)c->ncell + 1) * sizeof(int32_t), c->stream));
@@ -65,6 +66,7 @@ int set_list_skin(Ctx *c, double skin) {
     if (rc) return rc;
     rc = upload_tables(c);
     if (rc) return rc;
+    c->uploaded = true;
     c->binned = false;
     c->epoch++;
     return dem_list_request_rebuild(c);

@@ -1645,6 +1645,14 @@ __global__ void k_set_one(int32_t *p) { *p = 1; }
 
 }  // namespace
 
+int near_reserve(Ctx *c) {
+    if (c->posf && c->near) return PE_B200_OK;
+    const size_t n = (size_t)std::max<int64_t>(c->n, 1);
+    if (!c->posf) PEB_CUDA(c, dmalloc(c, &c->posf, n * sizeof(float4)));
+    PEB_CUDA(c, dmalloc(c, &c->near, n * (1 + kNear) * sizeof(int32_t)));
+    return PE_B200_OK;
+}
+
 namespace {
 // the sort of the current state, with the FP32 position copy of the default grid form
 int dem_sort(Ctx *c, bool with_pos) {
@@ -1652,9 +1660,9 @@ int dem_sort(Ctx *c, bool with_pos) {
         const int rc = grid_bin_current(c);
         if (rc) return rc;
     }
-    if (with_pos && !c->posf) {
-        PEB_CUDA(c, dmalloc(c, &c->posf, (size_t)c->n * sizeof(float4)));
-        PEB_CUDA(c, dmalloc(c, &c->near, (size_t)c->n * (1 + kNear) * sizeof(int32_t)));
+    if (with_pos) {
+        const int rc = near_reserve(c);
+        if (rc) return rc;
     }
     return grid_sort(c, with_pos);
 }
@@ -1819,6 +1827,7 @@ int list_capacity_check(Ctx *c) {
             const int64_t cap = std::max<int64_t>(2 * L.cap, need + need / 4 + 1024);
             dfree(c, L.idx);
             L.idx = nullptr;
+            L.cap = 0;   // without a buffer no list fits, and the steps search the grid
             PEB_CUDA(c, dmalloc(c, &L.idx, (size_t)cap * sizeof(int32_t)));
             L.cap = cap;
             c->epoch++;

@@ -447,6 +447,7 @@ int set_list_skin(Ctx *c, double skin);
 int set_tuning(Ctx *c, const Tuning &t, double skin);
 int autotune(Ctx *c, double dt, int32_t trial, pe_b200_tuning *out);
 int dem_step(Ctx *c, double dt);
+int near_reserve(Ctx *c);   // the grid step's position copy and candidate lists
 int dem_search(Ctx *c);   // sort and candidate lists of the current state, without a step
 int adjoint_forward(Ctx *c, int32_t nsteps, double dt, int32_t every);
 int adjoint_backward(Ctx *c, const double *gx, const double *gv, const double *gw, double *ox,

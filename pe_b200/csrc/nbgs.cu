@@ -2044,7 +2044,7 @@ __global__ void k_integrate(int64_t n, double dt, double drag, int has_drag, Bod
 }
 
 // ---- buffers -------------------------------------------------------------------------------
-int nbgs_alloc(Ctx *c, int64_t cap) {
+int nbgs_alloc_buffers(Ctx *c, int64_t cap) {
     NbgsBuf &b = c->nb;
     const size_t es = (c->p.precision == PE_B200_FP64) ? 8 : 4;
     const int64_t n = std::max<int64_t>(c->n, 1);
@@ -2122,6 +2122,14 @@ int nbgs_alloc(Ctx *c, int64_t cap) {
         PEB_CUDA(c, cudaMemsetAsync(b.bar2, 0, 2 * sizeof(unsigned int), c->stream));
     }
     return PE_B200_OK;
+}
+
+// the buffers of a hard-contact step for `cap` contacts; after a failure there are none, so that the
+// next step starts from the beginning instead of on those that were made
+int nbgs_alloc(Ctx *c, int64_t cap) {
+    const int rc = nbgs_alloc_buffers(c, cap);
+    if (rc) nbgs_free(c);
+    return rc;
 }
 
 template <typename T>
