@@ -1679,9 +1679,10 @@ namespace {
 // own step run on the side stream beside the spheres' sort, candidate lists and forces, which they
 // do not depend on: 110,592 spheres with 1,000 boxes took 160 us a step one after the other.  The
 // context's stream waits for the side stream before the step ends, so nothing else ever runs
-// beside it; without a side stream everything runs on the context's.
+// beside it; without a side stream, and while the stage timers run (they keep the stages apart),
+// everything runs on the context's.
 int dem_step_boxes(Ctx *c, double dt) {
-    const bool fork = split_streams(c);
+    const bool fork = !c->prof && split_streams(c);
     cudaStream_t side = fork ? c->side : c->stream;
     auto order = [&](cudaEvent_t ev, cudaStream_t first, cudaStream_t then) -> int {
         if (!fork) return PE_B200_OK;
@@ -1701,9 +1702,10 @@ int dem_step_boxes(Ctx *c, double dt) {
         rc = order(c->ev_join, side, c->stream);           // geometry -> forces on the spheres
         if (!rc) rc = order(c->ev_sort, c->stream, side);  // sort -> the boxes' step
         if (!rc) rc = mbox_dem_boxes(c, dt, side);
-        if (!rc && c->n > 0 && lists) rc = launch_near(c);
+        // beside the boxes' step; otherwise with the forces, as in a step without boxes
+        if (!rc && c->n > 0 && lists && fork) rc = launch_near(c);
         if (!rc) rc = mbox_dem_on_spheres(c);
-        if (!rc && c->n > 0) rc = launch_dem<double>(c, dt, lists);   // boxes: FP64 only
+        if (!rc && c->n > 0) rc = launch_dem<double>(c, dt, fork);   // boxes: FP64 only
         return rc ? rc : order(c->ev_join, side, c->stream);
     };
     const int rc = body();
