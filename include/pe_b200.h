@@ -249,8 +249,10 @@ typedef struct {
     double ms_per_step;      /* pe_b200_autotune: measured time of the winner; else -1 */
     int32_t variants;        /* output: number of launch shapes */
     int32_t nbgs_sweeps;     /* HCSITS sweeps: 0 automatic (a block for up to 768 contacts of a
-                                sphere scene, else each contact waits for its two bodies only, all
-                                in one cooperative grid), 1 one thread-block cluster with hardware
+                                sphere scene, or with moving boxes 1,100 without friction and 96
+                                with it; else each contact waits for its two bodies only, all in
+                                one cooperative grid, where its buffers find room: 80 bytes a
+                                contact in mixed precision, 144 in FP64), 1 one thread-block cluster with hardware
                                 barriers, 2 one cooperative grid with barriers through global
                                 memory, 3 one launch per colour, 4 one thread block with
                                 __syncthreads between colours (when every colour fits it), 5 one

@@ -741,7 +741,9 @@ __device__ void box_advance(const BoxArgs &a, int32_t m, V v, V w, double dt, do
 // one block per moving box: its contact forces, then BoxTrait::move (boxtrait/Default.h:149-220).
 // Bound: the chain of its phases (a few thousand dependent cycles each), so residency counts for
 // more than registers: 40 steps of 110,592 spheres and 1,000 boxes with their transfers took 5.64
-// ms at 190 registers (two blocks per SM), 5.39 with three blocks, 5.05 with four, 4.86 with six.
+// ms at 190 registers (two blocks per SM), 5.39 with three blocks, 5.05 with four, 4.86 with six,
+// although six leave 80 registers and spill: 2.8 KB of stores and 8.4 KB of loads a thread, which
+// the L1 serves behind the chain.
 __global__ void __launch_bounds__(kBoxBlk, 6) k_box_dem(BoxArgs a, double gx, double gy, double gz,
                                                      double dt, double drag, int has_drag,
                                                      double *xo, double *qo, double *vo,

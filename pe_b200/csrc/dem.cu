@@ -1044,7 +1044,8 @@ __device__ __forceinline__ bool steps_sync(unsigned int *words, unsigned int b, 
 // own state, mark and list range stay in registers, a step reads only its partners' records and
 // ends at one grid barrier (and the rebuild's own when one is due).  Each step reads one state
 // buffer and writes the other.  base: barriers of the launches before (words[3]).
-// Bound: the barrier (about 1 us) and the chain of a sphere's own dependent operations.  us per step
+// Bound: the barrier (about 1 us) and the chain of a sphere's own dependent operations (4,096 spheres:
+// 13% of the issue slots, 1% of the L2's throughput).  us per step
 // (two kernels per step, replayed / this): mostly apart, mixed 2,000 spheres 4.1 / 2.4, 30,000 4.8 /
 // 2.9, 100,000 5.7 / 3.9; FP64 30,000 5.0 / 2.7, 75,000 5.7 / 3.3; in contact, mixed 2,197 10.3 / 9.4,
 // 97,336 20.2 / 14.2; FP64 29,791 12.0 / 10.2; 32 scenes of 70,000 spheres in all 9.9 / 7.0; 4,096 on
@@ -1562,7 +1563,10 @@ int launch_rebuild_contacts(Ctx *c, const DemArgs<VT> &a, bool ovl, int *fused) 
         // per SM (405,224 spheres in contact: 62 us per step, 97 with one, 63 with three); in mixed
         // precision three (97,336 spheres in contact: 15.3 us, 18.4 with four, 25.5 with five;
         // 400,000 mostly apart: 10.3, 12.8, 17.4) until a fourth saves a whole pass over the
-        // spheres that outweighs its spills (1,048,576 in contact: 107 us with four, 115 with three).
+        // spheres that outweighs its spills.  us per step with three / four: in contact 592,704
+        // 66.0 / 65.7, 704,969 76.1 / 70.4, 1,061,208 107.9 / 100.9; mostly apart 600,000 13.2 /
+        // 13.6, 700,000 14.7 / 15.5, 1,048,576 25.8 / 25.6, 2,000,000 52.4 / 52.2: the line gives up
+        // 3-6% of a sparse step of 600,000 to a million for 7% of one in contact.
         constexpr int M = sizeof(VT) == 4 ? 3 : 2, MBIG = sizeof(VT) == 4 ? 4 : 2;
         const bool big = c->n >= 600000;
         if (one)
@@ -1865,7 +1869,8 @@ int list_step_any(Ctx *c, double dt) {
     return (c->p.precision == PE_B200_FP64) ? list_step<double>(c, dt) : list_step<float>(c, dt);
 }
 
-// largest scene whose steps run as one kernel
+// largest scene whose steps run as one kernel: three blocks of 256 threads on each of 148 SMs; the
+// launch tests the grid that is resident itself, this keeps larger scenes from asking at every call
 constexpr int64_t kStepsMax = 113664;
 
 void graph_key(const Ctx *c, const void *key[12]) {

@@ -11,8 +11,10 @@
 //                           walls never conflict: infinite mass)
 //   contact cache           frame n,t,o; ERP-scaled distance; Delassus block D, D^-1, 1/D_nn,
 //                           (D_to)^-1 (HCSITS.h:1741-1820), stored in colour-sorted order
-//   sweeps                  max_iterations x colours: each colour is a conflict-free parallel
-//                           Gauss-Seidel sweep (relaxInelasticFrictionlessContacts :2039-2105,
+//   sweeps                  max_iterations x colours of conflict-free Gauss-Seidel updates; each
+//                           waits only for its two bodies' updates of the colours before it
+//                           (k_sweeps_flow), or colours are swept one by one in a block, a
+//                           cluster or a grid (relaxInelasticFrictionlessContacts :2039-2105,
 //                           relaxApproximateInelasticCoulombContactsByDecoupling :2129-2304)
 //   integrate               x += (v'+dv) dt, quaternion, drag, store v, w (HCSITS.h:4135-4190)
 // Colour order replaces pe's detection order; only converged frictionless velocities are
@@ -462,9 +464,10 @@ __global__ void k_adj_fill(const int32_t *ncp, const int32_t *dd, const int32_t 
 // The guard of a step queued without the host: more contacts than the step was planned for
 // (the buffers' capacity, or none for a step planned without contacts) abort the rest of the
 // call (its steps leave the state as it is); the largest count is recorded (k_plan).  For a step
-// planned without contacts, in one launch instead of count, scan and plan: a sphere with any contact aborts the call's remaining steps (they are repeated with
-// the contact stages, which record the counts).  dd[kDdNc] stays 0 from the last step that
-// counted (it found none, or this plan would not have been chosen).
+// planned without contacts, in one launch instead of count, scan and plan: a sphere with any contact
+// aborts the call's remaining steps (they are repeated with the contact stages, which record the
+// counts).  dd[kDdNc] stays 0 from the last step that counted (it found none, or this plan would not
+// have been chosen).
 __global__ void k_any_contact(int64_t n, VisitArgs a, int32_t *dd) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n || dd[kDdAbort]) return;
@@ -2890,9 +2893,11 @@ int nbgs_step_t(Ctx *c, double dt, bool queued) {
     // the sweeps without barriers may run: k_cache writes the bodies' contacts in colour order
     // (over the colouring's adjacency, which it no longer needs)
     // Host-driven steps with fewer contacts stay in one block, whose hops through shared memory are
-    // shorter while it has few contacts to run: stacks of boxes, us per step (this / one block)
-    // without friction 2x2x2 1594 / 1199, 5x5x5 4245 / 4055, 6x6x6 5133 / 5745; with friction 3x3x3
-    // (93 contacts at the end) 3260 / 3152, 2x4x4 (145) 3373 / 3501, 6x6x6 6242 / 7910.
+    // shorter while it has few contacts to run.  18 stacks of boxes, 4 steps of 100 sweeps, us per
+    // step (this / one block) by the contacts at the end: without friction 36 1688 / 1187, 277 3968
+    // / 3321, 424 4111 / 3682, 607 4086 / 3859, 736 4566 / 4390, 1422 5598 / 6145 (one block is
+    // ahead by 4-30% in all 17 up to 736); with friction 15 1595 / 1430, 56 2806 / 2621, 29 to 297
+    // within 2% of one another, 370 5320 / 5683, 489 4849 / 5274, 1360 7148 / 8971.
     const int64_t flow_min = !gen ? kCompactMax
                              : c->p.relaxation_model == PE_B200_INELASTIC_FRICTIONLESS ? 1100 : 96;
     int32_t *flow_adj = nullptr;
