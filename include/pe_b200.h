@@ -252,8 +252,8 @@ typedef struct {
                                 sphere scene, or with moving boxes 1,100 without friction and 96
                                 with it; else each contact waits for its two bodies only, all in
                                 one cooperative grid, where its buffers find room: 80 bytes a
-                                contact in mixed precision, 144 in FP64), 1 one thread-block cluster with hardware
-                                barriers, 2 one cooperative grid with barriers through global
+                                contact in mixed precision, 144 in FP64), 1 one thread-block cluster
+                                with hardware barriers, 2 one cooperative grid with barriers through global
                                 memory, 3 one launch per colour, 4 one thread block with
                                 __syncthreads between colours (when every colour fits it), 5 one
                                 cluster with the bodies' records in its distributed shared memory
@@ -266,8 +266,8 @@ typedef struct {
                                 and 2 by size, precision and list density, and runs the steps of
                                 small scenes in one kernel; 0 the marked spheres' forces, then the
                                 integration of every sphere; 1 the marked spheres (forces and
-                                integration) on a second stream beside the integration of the others; 2 the same
-                                overlap on one stream: the kernel that checks for (and runs) the
+                                integration) on a second stream beside the integration of the others;
+                                2 the same overlap on one stream: the kernel that checks for (and runs) the
                                 rebuild lets the integration of the unmarked spheres start, then
                                 computes and integrates the marked ones (orientation tracking
                                 runs form 0).  All forms give the same results */

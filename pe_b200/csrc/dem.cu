@@ -1886,7 +1886,8 @@ void graph_key(const Ctx *c, const void *key[12]) {
 // began).
 bool steps_fit_kernel(const Ctx *c, int32_t steps) {
     return c->tune.dem_split < 0 && c->tune.rebuild_per_sm >= 0 && !c->nl.steps_off &&
-           !c->nl.coop_disabled && !c->prof && (steps & 1) == 0 && !c->p.track_orientation && c->p.force_model == 0 && c->n <= kStepsMax;
+           !c->nl.coop_disabled && !c->prof && (steps & 1) == 0 && !c->p.track_orientation &&
+           c->p.force_model == 0 && c->n <= kStepsMax;
 }
 
 template <typename VT>

@@ -3203,7 +3203,8 @@ bool nbgs_flow_free(Ctx *c) {
     NbgsBuf &b = c->nb;
     if (!b.flow) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        return false;
     nbgs_graph_free(c);
     dfree(c, b.flow);
     b.flow = nullptr;
